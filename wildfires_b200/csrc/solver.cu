@@ -270,8 +270,7 @@ struct wf_ctx {
     } ploop[4] = {};
     int ploop_next = 0;
     int closure = 0;         // WF_CLOSURE_SMAGORINSKY / WF_CLOSURE_MLP
-    int *d_bcfix = nullptr;  // columns left to k_stage_bc
-    int nbcfix = 0;
+    int kcmax = 0;           // highest cut node
     void *coef = nullptr;    // [N] learned coefficient (stencil precision)
     float *d_theta = nullptr;
     int *d_closure_err = nullptr;   // raised by the closure kernel on a timed-out tensor-core wait
@@ -279,8 +278,17 @@ struct wf_ctx {
     double *d_rep = nullptr;        // checkpoint report scratch
     Dumper *dump = nullptr;         // asynchronous dumps (created by the first wf_dump_async)
     int tile = 0;                   // tile shape of the fused stage pass (index)
-    bool tile_set = false;          // chosen by the tuner, WF_STAGE_TILE or wf_set_stage_tile
-    int *d_kerr = nullptr;          // raised by a stage kernel whose bounded tile wait gave up
+    int *d_kerr = nullptr;          // raised by a stage kernel whose bounded wait for a plane gave up
+    // tiling of the fused pass for form plan_tile, and TMA tensor maps (CUtensorMap,
+    // 128 bytes) of the buffers a stage reads for the boxes of its tiles and rows
+    int plan_tile = -1;
+    StageGrid grid;
+    void *encode = nullptr;         // cuTensorMapEncodeTiled, or nullptr: no maps
+    struct TensorMaps {
+        const void *ptr = nullptr;
+        alignas(64) unsigned char tile[128], row[128];
+    } tmaps[4];
+    bool tile_set = false;          // chosen by choose_tile or wf_set_stage_tile
     // wf_upload_state_async: p is copied on `up` after the state's copy (event
     // ev_y) and completes ev_p; the step waits for ev_p just before its pressure
     // solve, every other user of p first makes the context stream wait for it
@@ -291,24 +299,12 @@ struct wf_ctx {
     // the host copy of one chunk runs on `up` while the other is converted on
     // the context stream; ev_copy / ev_conv order the two per buffer
     cudaEvent_t ev_copy[2] = {nullptr, nullptr}, ev_conv[2] = {nullptr, nullptr};
-    // FP32: TMA tensor maps (CUtensorMap, 128 bytes) of the state buffers a stage
-    // reads, for the boxes of 16-column (map[0]) and 8-column (map[1]) tiles
-    struct TensorMaps {
-        const void *ptr = nullptr;
-        alignas(64) unsigned char map[2][128];
-        bool ok[2] = {false, false};
-    } tmaps[4];
-    int ntmaps = 0;
-    // FP32: maps of y_n (either step buffer) and acc for the boxes of a tile's own
-    // cells, with which the stage kernel prefetches its RK operands into L2
-    TensorMaps cmaps[3];
-    int ncmaps = 0;
 };
 
 namespace wfs {
 
 wf_status finish_upload(wf_ctx *c);
-wf_status tune_tiles(wf_ctx *c);
+wf_status choose_tile(wf_ctx *c);
 
 // Order the context stream after a pressure copy of wf_upload_state_async that
 // may still be in flight (callers that read or write p other than the step).
@@ -321,18 +317,17 @@ wf_status settle_p(wf_ctx *c)
     return WF_OK;
 }
 
-// Kernel launches of one step: per stage the optional closure inference,
-// k_utau, k_stage_fused and, when some column needs it, k_stage_bc; five
-// pressure kernels per solve (variable density: plus the record reset, the
-// source's p-independent part and, per iteration, k_maxdiff_copy and
-// k_piter_next; counted for max_iter iterations, an upper bound when the
-// tolerance ends the loop early); the projection.
+// Kernel launches of one step: k_utau, per stage the optional closure inference,
+// k_stage_march and k_stage_edge; five pressure kernels per solve (variable
+// density: plus the record reset, the source's p-independent part and, per
+// iteration, k_maxdiff_copy and k_piter_next; counted for max_iter iterations, an
+// upper bound when the tolerance ends the loop early); the projection.
 int launches_per_step(const wf_ctx *c)
 {
-    const int per_stage = 2 + (c->nbcfix > 0 ? 1 : 0) + (c->closure ? 1 : 0);
+    const int per_stage = 2 + (c->closure ? 1 : 0);
     const int maxit = c->P.pressure_solver_iter > 0 ? c->P.pressure_solver_iter : 0;
     const int pressure = (c->P.variable_density != 0) ? 1 + (maxit > 0 ? 1 : 0) + 7 * maxit : 5;
-    return c->nstages * per_stage + pressure + 1;
+    return 1 + c->nstages * per_stage + pressure + 1;
 }
 
 // Failure injection (wf_inject_allocation_failure): the number of context
@@ -491,8 +486,24 @@ std::vector<double> krow_table(const Parameters &P, const double *z, const std::
         r[RDEL2] = Z(ZDELTA2, k);
         r[RZ] = z[k];
         r[RDD2] = pow(P.dx * P.dy * Z(ZDZ, k), 2.0 / 3.0);
+        if (k <= Nz - 3) {
+            const double A = z[k + 1] - z[k], B = z[k + 2] - z[k + 1];
+            r[RCUT1] = (A + B) * (A + B) / (B * (2 * A + B));
+            r[RCUT2] = A * A / (B * (2 * A + B));
+        }
     }
     return t;
+}
+
+// top-plane extrapolation f_{Nz-1} = w1 f_{Nz-2} - w2 f_{Nz-3} (pde.cu:79-86)
+template <class R> void top_weights(const Parameters &P, R &w1, R &w2)
+{
+    w1 = w2 = R(0);
+    if (!P.z || P.Nz < 3) return;
+    const int k = P.Nz - 1;
+    const double a1 = P.z[k] - P.z[k - 1], a2 = P.z[k - 1] - P.z[k - 2], den = a2 * (a2 + 2 * a1);
+    w1 = (R)((a2 + a1) * (a2 + a1) / den);
+    w2 = (R)(a1 * a1 / den);
 }
 
 template <class R> PhysR<R> make_physr(const Parameters &P)
@@ -516,6 +527,12 @@ template <class R> PhysR<R> make_physr(const Parameters &P)
     r.mu_Trho = (R)(P.mu / (P.T_inf * P.rho_inf));
     r.inv_Trho_cp = (R)(1.0 / (P.T_inf * P.rho_inf * P.c_p));
     r.H_C_cp = (R)(P.H_C / P.c_p);
+    r.dead[0] = (R)P.u_dead_nodes; r.dead[1] = (R)P.v_dead_nodes; r.dead[2] = (R)P.w_dead_nodes;
+    r.dead[3] = (R)P.T_dead_nodes; r.dead[4] = (R)P.Y_dead_nodes;
+    top_weights(P, r.top_w1, r.top_w2);
+    r.g_Tinf = (R)(P.g / P.T_inf);
+    r.two_inv_Trho = (R)(2.0 / (P.T_inf * P.rho_inf));
+    r.inv_Trho_Pr = (R)(1.0 / (P.T_inf * P.rho_inf * P.Pr));
     r.T_min = (R)P.T_min; r.T_max = (R)P.T_max; r.Y_min = (R)P.Y_min; r.Y_max = (R)P.Y_max;
     return r;
 }
@@ -537,14 +554,24 @@ Phys make_phys(const Parameters &P)
     ph.sutherland_conductivity = P.sutherland_conductivity;
     ph.variable_density = P.variable_density;
     ph.velocity_correction_fd = P.velocity_correction_fd;
-    if (P.z && P.Nz >= 3) {
-        const int k = P.Nz - 1;
-        const double a1 = P.z[k] - P.z[k - 1], a2 = P.z[k - 1] - P.z[k - 2];
-        const double den = a2 * (a2 + 2 * a1);
-        ph.top_w1 = (a2 + a1) * (a2 + a1) / den;
-        ph.top_w2 = a1 * a1 / den;
-    }
+    top_weights(P, ph.top_w1, ph.top_w2);
     return ph;
+}
+
+// Tiling and tensor maps of the fused stage pass for the context's block form.
+void plan_stage(wf_ctx *c)
+{
+    const int prec = c->prec == WF_FP64 ? 0 : 1;
+    c->grid = stage_plan(prec, c->tile, c->Nx, c->Ny, c->Nz);
+    c->plan_tile = c->tile;
+    const void *bufs[4] = {c->ybuf[0], c->ybuf[1], c->Xa, c->Xb};
+    for (int b = 0; b < 4; b++) {
+        auto &m = c->tmaps[b];
+        m.ptr = nullptr;
+        if (bufs[b] && stage_tensor_map(m.tile, bufs[b], prec, c->Nx, c->Ny, c->Nz, c->grid.tj + 4, c->encode) &&
+            stage_tensor_map(m.row, bufs[b], prec, c->Nx, c->Ny, c->Nz, 1, c->encode))
+            m.ptr = bufs[b];
+    }
 }
 
 template <class R> StageArgs<R> stage_args(wf_ctx *c, const void *X, const void *yn, void *Xout, int stage)
@@ -567,20 +594,19 @@ template <class R> StageArgs<R> stage_args(wf_ctx *c, const void *X, const void 
     a.theta = c->d_theta;
     a.closure_err = c->d_closure_err;
     a.closure_wait = c->closure_wait;
-    a.bcfix = c->d_bcfix;
-    a.nbcfix = c->nbcfix;
-    a.kerr = c->d_kerr;
-    a.tmap[0] = a.tmap[1] = nullptr;
-    for (int q = 0; q < c->ntmaps; q++)
-        if (c->tmaps[q].ptr == X)
-            for (int b = 0; b < 2; b++) a.tmap[b] = c->tmaps[q].ok[b] ? c->tmaps[q].map[b] : nullptr;
-    for (int b = 0; b < 2; b++) a.pmap_yn[b] = a.pmap_acc[b] = nullptr;
-    for (int q = 0; q < c->ncmaps; q++)
-        for (int b = 0; b < 2; b++) {
-            if (c->cmaps[q].ptr == yn) a.pmap_yn[b] = c->cmaps[q].ok[b] ? c->cmaps[q].map[b] : nullptr;
-            if (c->cmaps[q].ptr == c->acc) a.pmap_acc[b] = c->cmaps[q].ok[b] ? c->cmaps[q].map[b] : nullptr;
-        }
+    a.kcmax = c->kcmax;
+    a.have_utau = c->method != 3 && stage > 1;
+    a.make_utau = c->method != 3 && stage < c->nstages;
     a.tile = c->tile;
+    a.kerr = c->d_kerr;
+    if (c->plan_tile != c->tile) plan_stage(c);
+    a.grid = c->grid;
+    a.tmap[0] = a.tmap[1] = nullptr;
+    for (const auto &m : c->tmaps)
+        if (m.ptr && m.ptr == X) {
+            a.tmap[0] = m.tile;
+            a.tmap[1] = m.row;
+        }
     const double dt = c->P.dt;
     if (c->method == 0) a.a_next = dt;
     else if (c->method == 1) a.a_next = (stage == 1) ? dt : 0.5 * dt;
@@ -1093,59 +1119,21 @@ wf_status wf_create(const Parameters *P, int precision, wf_ctx **out)
     cudaError_t e = (precision == WF_FP64) ? poisson_set_attributes<double>() : poisson_set_attributes<float>();
     if (e == cudaSuccess) e = (precision == WF_FP64) ? stage_set_attributes<double>() : stage_set_attributes<float>();
     if (e != cudaSuccess) { set_error("wf_create: %s", cudaGetErrorString(e)); return fail(WF_ERR_CUDA); }
-    {
-        // columns whose cut node (or, for every column, the top plane) the
-        // fused stage pass cannot complete within one z-tile
-        const int KZ = stage_tile_planes(precision);
-        const bool top_ok = (Nz - 1) / KZ == (Nz - 3) / KZ;
-        std::vector<int> fix;
-        for (int col = 0; col < Nx * Ny; col++) {
-            const int kc = c->hcut[col];
-            if (!top_ok || kc / KZ != (kc + 2) / KZ) fix.push_back(col);
-        }
-        c->nbcfix = (int)fix.size();
-        if (!fix.empty() && (st = upload(c, &c->d_bcfix, fix.data(), fix.size()))) return fail(st);
-    }
+    for (int col = 0; col < Nx * Ny; col++)
+        if (c->hcut[col] > c->kcmax) c->kcmax = c->hcut[col];
     e = cudaMemsetAsync(c->p, 0, sizeof(double) * c->N, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) { set_error("wf_create: %s", cudaGetErrorString(e)); return fail(WF_ERR_CUDA); }
     if ((st = dev_alloc(c, (void **)&c->d_kerr, sizeof(int)))) return fail(st);
     e = cudaMemset(c->d_kerr, 0, sizeof(int));
     if (e != cudaSuccess) { set_error("wf_create: %s", cudaGetErrorString(e)); return fail(WF_ERR_CUDA); }
-    if (precision != WF_FP64 && !(getenv("WF_NO_TMA") && atoi(getenv("WF_NO_TMA")))) {
-        // tensor maps for the tile loads of the FP32 stage kernel, one per state
-        // buffer a stage can read; without them (column length not a multiple
-        // of 4, or no driver entry point) the tiles are loaded by cp.async
-        void *encode = nullptr;
+    if (!(getenv("WF_NO_TMA") && atoi(getenv("WF_NO_TMA")))) {
+        // for the tensor maps; without it the stage kernel copies its planes by cp.async
         cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &encode, cudaEnableDefault, &q) != cudaSuccess ||
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &c->encode, cudaEnableDefault, &q) != cudaSuccess ||
             q != cudaDriverEntryPointSuccess)
-            encode = nullptr;
+            c->encode = nullptr;
         cudaGetLastError();
-        const void *bufs[4] = {c->ybuf[0], c->ybuf[1], c->Xa, c->Xb};
-        for (int b = 0; b < 4 && encode; b++) {
-            if (!bufs[b]) continue;
-            auto &m = c->tmaps[c->ntmaps];
-            m.ok[0] = stage_tensor_map(m.map[0], (const float *)bufs[b], Nx, Ny, Nz, 8, 16, encode);
-            m.ok[1] = stage_tensor_map(m.map[1], (const float *)bufs[b], Nx, Ny, Nz, 8, 8, encode);
-            if (m.ok[0] || m.ok[1]) {
-                m.ptr = bufs[b];
-                c->ntmaps++;
-            }
-        }
-        // the RK operands' cell boxes (WF_NO_PREFETCH=1: none, for comparisons)
-        const void *cbufs[3] = {c->ybuf[0], c->ybuf[1], c->acc};
-        const bool no_pf = getenv("WF_NO_PREFETCH") && atoi(getenv("WF_NO_PREFETCH"));
-        for (int b = 0; b < 3 && encode && !no_pf; b++) {
-            if (!cbufs[b]) continue;
-            auto &m = c->cmaps[c->ncmaps];
-            m.ok[0] = stage_cell_map(m.map[0], (const float *)cbufs[b], Nx, Ny, Nz, 8, 16, encode);
-            m.ok[1] = stage_cell_map(m.map[1], (const float *)cbufs[b], Nx, Ny, Nz, 8, 8, encode);
-            if (m.ok[0] || m.ok[1]) {
-                m.ptr = cbufs[b];
-                c->ncmaps++;
-            }
-        }
     }
     c->launches = launches_per_step(c);
     *out = c;
@@ -1260,17 +1248,16 @@ wf_status finish_upload(wf_ctx *c)
     return st == WF_ERR_NAN ? WF_OK : st;
 }
 
-// Tile shape of the fused stage pass for this context.  WF_STAGE_TILE=TIxTJ in
-// the environment forces a shape; otherwise, when more than one shape is
-// compiled, each is timed on the context's own grid and current state (a
-// stage that stores k_s into a scratch buffer, so the state is untouched: one
-// warm-up launch, then enough launches for about 2 ms, at least 3) and the
-// fastest kept.  Every shape gives
-// bit-identical results: a cell's arithmetic does not depend on the tiling.
-template <class R> wf_status tune_tiles_impl(wf_ctx *c)
+// Block form of the fused stage pass for this context: WF_STAGE_TILE=TIxTJ[/threads]
+// in the environment forces one, otherwise the one stage_default_form gives.
+// Every form gives bit-identical results: a cell's arithmetic does not depend
+// on the tiling.
+wf_status choose_tile(wf_ctx *c)
 {
-    const int prec = c->prec == WF_FP64 ? 0 : 1, count = stage_tile_count(prec);
+    if (c->tile_set) return WF_OK;
     c->tile_set = true;
+    const int prec = c->prec == WF_FP64 ? 0 : 1, count = stage_tile_count(prec);
+    c->tile = stage_default_form(prec);
     if (const char *env = getenv("WF_STAGE_TILE")) {
         int ti = 0, tj = 0, nt = 0;
         const int got = sscanf(env, "%dx%d/%d", &ti, &tj, &nt);   // TIxTJ, optionally /threads
@@ -1278,53 +1265,15 @@ template <class R> wf_status tune_tiles_impl(wf_ctx *c)
             for (int q = 0; q < count; q++) {
                 int a = 0, b = 0, n = 0;
                 stage_tile_shape(prec, q, &a, &b, &n);
-                if (a == ti && b == tj && (got < 3 || n == nt)) { c->tile = q; return WF_OK; }
+                if (a == ti && b == tj && (got < 3 || n == nt)) {
+                    c->tile = q;
+                    return WF_OK;
+                }
             }
         set_error("WF_STAGE_TILE=%s is not a compiled tile shape", env);
         return WF_ERR_ARG;
     }
-    if (count < 2) return WF_OK;
-    void *in = c->ybuf[c->cur], *scratch = c->Xa ? c->Xa : c->ybuf[1 - c->cur];
-    const int saved = c->method;
-    c->method = 3;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
-        if (e0) cudaEventDestroy(e0);
-        c->method = saved;
-        set_error("stage tile tuning: %s", cudaGetErrorString(cudaGetLastError()));
-        return WF_ERR_CUDA;
-    }
-    float best = 1e30f;
-    int pick = 0;
-    cudaError_t err = cudaSuccess;
-    for (int q = 0; q < count && !err; q++) {
-        c->tile = q;
-        const StageArgs<R> a = stage_args<R>(c, in, in, scratch, 1);
-        float ms = 0.0f;
-        int reps = 1;
-        for (int pass = 0; pass < 2 && !err; pass++) {   // pass 0 warms up and sizes pass 1
-            err = cudaEventRecord(e0, c->stream);
-            for (int r = 0; r < reps && !err; r++) err = launch_stage<R>(a, c->stream);
-            if (!err) err = cudaEventRecord(e1, c->stream);
-            if (!err) err = cudaEventSynchronize(e1);
-            if (!err) err = cudaEventElapsedTime(&ms, e0, e1);
-            if (pass == 0) reps = ms > 0.0f ? (int)fminf(fmaxf(2.0f / ms, 3.0f), 64.0f) : 3;
-        }
-        ms /= (float)reps;
-        if (!err && ms < best) { best = ms; pick = q; }
-    }
-    c->method = saved;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    c->tile = pick;
-    if (err) { set_error("stage tile tuning: %s", cudaGetErrorString(err)); return WF_ERR_CUDA; }
     return WF_OK;
-}
-
-wf_status tune_tiles(wf_ctx *c)
-{
-    if (c->tile_set) return WF_OK;
-    return c->prec == WF_FP64 ? tune_tiles_impl<double>(c) : tune_tiles_impl<float>(c);
 }
 }  // namespace wfs
 
@@ -1348,7 +1297,7 @@ wf_status wf_step(wf_ctx *c, int nsteps)
     const NvtxRange range("wf_step");
     if (!c || nsteps < 0) { set_error("wf_step: invalid argument"); return WF_ERR_ARG; }
     if (nsteps > 0) {
-        const wf_status st = tune_tiles(c);
+        const wf_status st = choose_tile(c);
         if (st) return st;
     }
     for (int q = 0; q < nsteps; q++) {
@@ -1397,7 +1346,7 @@ wf_status wf_synchronize(wf_ctx *c)
         WF_TRY_CUDA(cudaMemcpy(&herr, c->d_kerr, sizeof(int), cudaMemcpyDeviceToHost));
         if (herr) {
             WF_TRY_CUDA(cudaMemset(c->d_kerr, 0, sizeof(int)));
-            set_error("wf_synchronize: a stage kernel's wait for its tile load timed out");
+            set_error("wf_synchronize: a stage kernel's wait for a state plane timed out");
             return WF_ERR_CUDA;
         }
     }
@@ -1726,7 +1675,7 @@ wf_status wf_ensemble_step(wf_ensemble *e, int nsteps)
     const NvtxRange range("wf_ensemble_step");
     if (!e || nsteps < 0) { set_error("wf_ensemble_step: invalid argument"); return WF_ERR_ARG; }
     for (wf_ctx *c : e->m) {
-        const wf_status st = nsteps > 0 ? tune_tiles(c) : WF_OK;
+        const wf_status st = nsteps > 0 ? choose_tile(c) : WF_OK;
         if (st) return st;
     }
     for (int q = 0; q < nsteps; q++) {

@@ -4,13 +4,15 @@
 // Smagorinsky SGS terms, boundary/IBM rules) and folds the RK combination into
 // the same pass (reference solver.cu:14-93, utils.cu:14-21), so no k-buffer is
 // ever stored:
-//   k_utau        : per column, wall friction velocity from the k = 0 plane;
-//   k_stage_fused : per tile of cells in shared memory, the SGS inputs on the
-//                   tile and its halo, then advection + diffusion + forces +
-//                   reaction + SGS divergence and the acc / X_{s+1} updates of
-//                   every cell the boundary rules do not overwrite;
-//   k_stage_bc    : per column, the boundary/IBM values of k_s (cut node, top,
-//                   dead nodes) and their RK updates.
+//   k_utau        : per column, wall friction velocity from the k = 0 plane (first
+//                   stage; k_stage_edge leaves it for the following ones);
+//   k_stage_march : per tile of cells, plane by plane along x in shared memory, the
+//                   SGS inputs of the tile and its frame, then advection +
+//                   diffusion + forces + reaction + SGS divergence and the acc /
+//                   X_{s+1} updates of every cell the boundary rules do not
+//                   overwrite;
+//   k_stage_edge  : the fuel, the boundary/IBM values of k_s (cut node, top) and
+//                   their RK updates.
 // The right-hand side of cells on the walls (k = 0, k = Nz-1) and below the
 // cut node is never used by the reference (boundary_conditions overwrites it,
 // pde.cu:58-97), so the fused pass evaluates interior stencils only.
@@ -21,6 +23,8 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "stage_common.cuh"
 
 namespace wf {
@@ -30,6 +34,20 @@ namespace {
 // ---------------------------------------------------------------------------
 // wall friction velocity of every column from its k = 0 plane
 // (pde.cu:767-772: tau_w = sqrt((mu uz)^2 + (mu vz)^2), u_tau = sqrt(tau_w/rho))
+template <class R> __device__ __forceinline__ R utau_of(const StageArgs<R> &a, const R (&u)[3], const R (&v)[3], R T)
+{
+    const int Nz = a.g.Nz;
+    const R w0 = (R)a.g.zc[ZF0 * Nz], w1 = (R)a.g.zc[ZF1 * Nz], w2 = (R)a.g.zc[ZF2 * Nz];
+    const R uz = w0 * u[0] + w1 * u[1] + w2 * u[2];
+    const R vz = w0 * v[0] + w1 * v[1] + w2 * v[2];
+    const R rho = fdiv(a.pr.Trho, T);
+    R mu = a.pr.mu;
+    if (a.ph.sutherland_viscosity == 1)
+        mu = R(1.716e-5) * rpow(T / R(273.15), R(1.5)) * (R(273.15) + R(110.4)) / (T + R(110.4));
+    const R a1 = mu * uz, a2 = mu * vz;
+    return rsqrt_(fdiv(rsqrt_(a1 * a1 + a2 * a2), rho));
+}
+
 template <class R>
 __global__ void __launch_bounds__(128) k_utau(const StageArgs<R> a)
 {
@@ -38,148 +56,125 @@ __global__ void __launch_bounds__(128) k_utau(const StageArgs<R> a)
     if (col >= g.Nx * g.Ny) return;
     const int Nz = g.Nz, N = g.N;
     const R *X = a.X + (size_t)col * Nz;
-    const R w0 = (R)g.zc[ZF0 * Nz], w1 = (R)g.zc[ZF1 * Nz], w2 = (R)g.zc[ZF2 * Nz];
-    const R uz = w0 * X[0] + w1 * X[1] + w2 * X[2];
-    const R vz = w0 * X[N] + w1 * X[N + 1] + w2 * X[N + 2];
-    const R T = X[3 * (size_t)N];
-    const R rho = fdiv(a.pr.Trho, T);
-    R mu = a.pr.mu;
-    if (a.ph.sutherland_viscosity == 1)
-        mu = R(1.716e-5) * rpow(T / R(273.15), R(1.5)) * (R(273.15) + R(110.4)) / (T + R(110.4));
-    const R a1 = mu * uz, a2 = mu * vz;
-    const R tau_w = rsqrt_(a1 * a1 + a2 * a2);
-    a.utau[col] = rsqrt_(fdiv(tau_w, rho));
+    const R u[3] = {X[0], X[1], X[2]}, v[3] = {X[N], X[N + 1], X[N + 2]};
+    a.utau[col] = utau_of(a, u, v, X[3 * (size_t)N]);
 }
 
-// Shared-memory tile of one stage: TI x TJ x KZ cells, state halo 2 (4 fields)
-// and SGS-input halo 1 (8 fields).  Offsets are relative to the tile origin;
-// (ii, jj, kk) in [-2, T+1] for the state and [-1, T] for the rest.  Both
-// arrays are stored j-fastest with a row stride of TJ+4: a warp covering
-// 8 consecutive k x 4 consecutive j then touches 32 distinct banks (FP32).
-// In FP32 the state is stored as two arrays of pairs, (u, v) and (w, T), so
-// one 8-byte load brings two fields and the pair arithmetic runs on FFMA2;
-// each half-warp (4 k x 4 j) of an 8-byte load then covers the 16 bank pairs.
-// The fuel fraction is read from global memory where a column has fuel.
-template <class R, int TI, int TJ, int KZ> struct Tile {
-    static constexpr int SI = TI + 4, SJ = TJ + 4, SK = KZ + 4, SR = SI * SJ * SK;
-    static constexpr int GI = TI + 2, GJ = TJ + 2, GK = KZ + 2, GJP = SJ, GR = GI * GK * GJP;
-    static constexpr bool PAIRED = sizeof(R) == 4;
-    static constexpr int NCOL = GI * GJ, CELLS = TI * TJ * KZ;
-    static constexpr size_t up16(size_t b) { return (b + 15) / 16 * 16; }
-    static constexpr size_t O_KR = up16(sizeof(R) * 4 * (size_t)SR);
-    static constexpr size_t O_TOPO = O_KR + up16(sizeof(R) * (size_t)GK * KROW);
-    static constexpr size_t O_UT = O_TOPO + up16(sizeof(double) * (size_t)NCOL);
-    static constexpr size_t O_NZY = O_UT + up16(sizeof(R) * (size_t)NCOL);
-    static constexpr size_t O_CUT = O_NZY + up16(sizeof(int) * (size_t)NCOL);
-    static constexpr size_t O_MISC = O_CUT + up16(sizeof(int) * (size_t)NCOL);   // mbarrier, flags
-    // the SGS buffer doubles as the staging area of the TMA box (512-byte aligned: 64-byte swizzle)
-    static constexpr size_t BUF = (O_MISC + 32 + 1023) / 1024 * 1024;
-    static constexpr size_t BOX = sizeof(float) * 4 * (size_t)SI * SJ * 16;   // one box, FP32 path
-    static constexpr size_t bytes() { return BUF + up16(sizeof(R) * 8 * (size_t)GR); }
-    R *st;         // [4][SR]  u, v, w, T
-    R *kr;         // [GK][KROW] z-stencil rows for k0-1 .. k0+KZ
-    double *ctopo; // [NCOL]   terrain height of the halo-1 columns
-    R *cut_;       // [NCOL]   wall friction velocity of the halo-1 columns
-    int *cnzy, *ccut;
-    R *gs;         // [8][GR]  mu_sgs, S11, S12, S13, S22, S23, S33, divU (shared by both buffers)
-    __device__ void bind(unsigned char *buf, R *sgs)
-    {
-        st = reinterpret_cast<R *>(buf);
-        kr = reinterpret_cast<R *>(buf + O_KR);
-        ctopo = reinterpret_cast<double *>(buf + O_TOPO);
-        cut_ = reinterpret_cast<R *>(buf + O_UT);
-        cnzy = reinterpret_cast<int *>(buf + O_NZY);
-        ccut = reinterpret_cast<int *>(buf + O_CUT);
-        gs = sgs;
-    }
-    __device__ static int s(int ii, int jj, int kk) { return ((ii + 2) * SK + (kk + 2)) * SJ + (jj + 2); }
-    __device__ static int q(int ii, int jj, int kk) { return ((ii + 1) * GK + (kk + 1)) * GJP + (jj + 1); }
-    __device__ static int cq(int ii, int jj) { return (ii + 1) * GJ + (jj + 1); }
-    // position of field f at tile offset sidx: pairs (u, v), (w, T) in FP32, planar in FP64
-    __device__ static int so(int f, int sidx) { return PAIRED ? (f >> 1) * 2 * SR + 2 * sidx + (f & 1) : f * SR + sidx; }
-    __device__ R &S(int f, int ii, int jj, int kk) { return st[so(f, s(ii, jj, kk))]; }
-    // pair pr (0: u, v; 1: w, T), FP32 only
-    __device__ float2 P(int pr, int ii, int jj, int kk) const
-    {
-        return reinterpret_cast<const float2 *>(st)[pr * SR + s(ii, jj, kk)];
-    }
-    __device__ R &G(int f, int ii, int jj, int kk) { return gs[f * GR + q(ii, jj, kk)]; }
-    __device__ R K(int kk, int e) const { return kr[(kk + 1) * KROW + e]; }
-};
+// ---------------------------------------------------------------------------
+// The fused stage pass.  A block owns a tile of TJ rows (j) x TK planes (k) of
+// cells and walks it along x, one x-plane per iteration; an interior thread owns
+// VW cells in k (FP32: 2, every operation on packed pairs; FP64: 1) of one row.
+// In iteration c it
+//   A. forms from the state planes c-2 .. c+2 in shared memory the SGS inputs of
+//      plane c (strain S', raw mu_sgs, the divergence source), the upwind
+//      advection, the Laplacians and the source terms;
+//   B. completes plane c-1: the SGS divergence from the SGS inputs of planes
+//      c-2, c-1 and c, and the RK update.
+// The fuel and the boundary cells (cut node, top) are k_stage_edge's; what
+// part B writes there is lost, and it leaves the k-values they need in a.bc.
+// State planes arrive three iterations ahead by TMA, one box per plane (one per
+// row where the tile's halo wraps around in y; in x the wrap is the choice of a
+// coordinate);
+// grids whose columns are no multiple of 16 bytes are copied by cp.async instead.
+// One barrier per plane.  FR further threads own the one-cell frame around the
+// tile, whose SGS inputs part B of the tile's edge reads.
+constexpr int kColRing = 8;   // x-planes of column tables kept (power of two)
+constexpr int kTileK = 32, kTileK2 = 24;   // planes of a tile at most: the two row lengths compiled
 
-// Asynchronous global -> shared copies (cp.async, sm_80+ PTX).  src_bytes 0
-// writes zeros without reading, which gives the tile its zero halo in z.
+// value of a thread's VW cells
+struct F2 {
+    float2 v;
+};
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) { return {__fadd2_rn(a.v, b.v)}; }
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return {__fmul2_rn(a.v, b.v)}; }
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return {__ffma2_rn(b.v, make_float2(-1.0f, -1.0f), a.v)}; }
+__device__ __forceinline__ F2 vfma(F2 a, F2 b, F2 c) { return {__ffma2_rn(a.v, b.v, c.v)}; }
+__device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
+template <class R> struct Vec;
+template <> struct Vec<float> {
+    using V = F2;
+    static constexpr int W = 2;
+};
+template <> struct Vec<double> {
+    using V = double;
+    static constexpr int W = 1;
+};
+template <class V> __device__ __forceinline__ V splat(float a) { return {make_float2(a, a)}; }
+template <class V> __device__ __forceinline__ V splat(double a) { return a; }
+__device__ __forceinline__ float el(const F2 &a, int e) { return e ? a.v.y : a.v.x; }
+__device__ __forceinline__ double el(double a, int) { return a; }
+__device__ __forceinline__ void set_el(F2 &a, int e, float x) { (e ? a.v.y : a.v.x) = x; }
+__device__ __forceinline__ void set_el(double &a, int, double x) { a = x; }
+__device__ __forceinline__ F2 vpos(F2 a) { return {make_float2(fmaxf(a.v.x, 0.0f), fmaxf(a.v.y, 0.0f))}; }
+__device__ __forceinline__ F2 vneg(F2 a) { return {make_float2(fminf(a.v.x, 0.0f), fminf(a.v.y, 0.0f))}; }
+__device__ __forceinline__ double vpos(double a) { return rmax(a, 0.0); }
+__device__ __forceinline__ double vneg(double a) { return rmin(a, 0.0); }
+__device__ __forceinline__ F2 vsqrt(F2 a) { return {make_float2(rsqrt_(a.v.x), rsqrt_(a.v.y))}; }
+__device__ __forceinline__ double vsqrt(double a) { return sqrt(a); }
+__device__ __forceinline__ F2 vdiv(F2 a, F2 b) { return {make_float2(fdiv(a.v.x, b.v.x), fdiv(a.v.y, b.v.y))}; }
+__device__ __forceinline__ double vdiv(double a, double b) { return a / b; }
+
+// per-k weights in shared memory, each a row over the tile's planes: upwind from
+// below (k-2, k-1, k) and from above (k, k+1, k+2), negated, the part of w each carries
+// (from below: max(w,0) WP + w WW, from above the rest of w), centred first
+// derivative, Smagorinsky length squared, centred second derivative (k-1, k+1),
+// height, spacing.  Weights apply to differences from the value at k.
+enum ZRow { ZB = 0, ZF = 3, ZWP = 6, ZWW, ZD1, ZL, ZD2, ZZ = ZD2 + 2, ZDZ, ZROW };
+// SGS inputs in shared memory
+enum GRow { G_MU, G_Q, G_S11, G_S12, G_S13, G_S22, G_S23, G_S33, GROW };
+
+// Shared memory of a block, in bytes from its start.  A row of the state holds
+// its four fields one after the other (the layout of a TMA box), KH planes of
+// halo on either side; consecutive cells are consecutive words, so every access
+// of a warp is free of bank conflicts.
+template <class R, int KW> struct StageSmem {
+    static constexpr uint32_t E = sizeof(R);
+    static constexpr int KH = 16 / E;                              // halo planes: a 16-byte boundary
+    static constexpr int PX = KW + 2 * KH, PG = KW + 4, RS = 6, RG = 3;
+    static constexpr uint32_t FX = PX * E;                         // one field of a row
+    static constexpr uint32_t ROW_S = 4 * FX;                      // a multiple of 128 bytes, as a box's start must be
+    static constexpr uint32_t FG = PG * E, ROW_G = GROW * FG;
+    static constexpr uint32_t FZ = PG * E;
+    uint32_t planeS, planeG;
+    uint32_t g0;            // start of the SGS ring
+    uint32_t zr;            // [ZROW][PG]
+    uint32_t wall;          // bottom and top: weights of the value beyond the wall (3) and of the second derivative (4)
+    uint32_t corr;          // V [2][2][TJ + 2]: second z derivative of T on the bottom and top wall; then a zero
+    uint32_t cidx;          // [kColRing][TJ + 2] int2: fuel top, cut node
+    uint32_t ctopo, cut_;   // [kColRing][TJ + 2] terrain height, wall friction velocity
+    uint32_t bnd;           // [2][TJ][2] highest terrain and least friction / A of the five columns around a cell
+    uint32_t zero;          // [2][TJ] int: which of them have no friction (bits: centre, x+, x-, y+, y-)
+    uint32_t bar;           // [RS] mbarriers of the state planes
+    uint32_t end;
+    __host__ __device__ explicit StageSmem(int tj)
+    {
+        planeS = (uint32_t)(tj + 4) * ROW_S;
+        planeG = (uint32_t)(tj + 2) * ROW_G;
+        g0 = RS * planeS;
+        bar = g0 + RG * planeG;
+        zr = bar + RS * 8;
+        wall = zr + ZROW * FZ;
+        corr = wall + 16 * E;
+        cidx = corr + (8 * (tj + 2) + 2) * E;
+        ctopo = cidx + kColRing * (tj + 2) * 8;
+        cut_ = ctopo + kColRing * (tj + 2) * E;
+        bnd = cut_ + kColRing * (tj + 2) * E;
+        zero = bnd + 4 * tj * E;
+        end = zero + 2 * tj * 4;
+    }
+    __device__ static uint32_t s(int jj, int kk) { return (uint32_t)(jj + 2) * ROW_S + (uint32_t)(kk + KH) * E; }
+    __device__ static uint32_t g(int jj, int kk) { return (uint32_t)(jj + 1) * ROW_G + (uint32_t)(kk + 2) * E; }
+    __device__ static uint32_t z(int kk) { return (uint32_t)(kk + 2) * E; }
+};
+extern __shared__ __align__(128) unsigned char stage_smem[];
+template <class T> __device__ __forceinline__ T &sh(uint32_t o) { return *reinterpret_cast<T *>(stage_smem + o); }
+
 template <int B>
-__device__ __forceinline__ void cp_async(void *dst, const void *src, bool valid)
+__device__ __forceinline__ void cp_async(uint32_t dst, const void *src, bool valid)
 {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    const unsigned d = (unsigned)__cvta_generic_to_shared(stage_smem) + dst;
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(B), "r"(valid ? B : 0)
                  : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Issue the copies of one tile's inputs into buffer t (one commit group).
-// Periodic in x and y (period N-1), zero outside 0..Nz-1 in z.
-template <class R, class TL, int NT>
-__device__ __forceinline__ void issue_tile(const StageArgs<R> &a, TL &t, int i0, int j0, int k0, bool state)
-{
-    const Geom &g = a.g;
-    const int Nx = g.Nx, Ny = g.Ny, Nz = g.Nz, N = g.N;
-    const R *__restrict__ X = a.X;
-    for (int c = threadIdx.x; c < TL::NCOL; c += NT) {
-        const int jj = c % TL::GJ - 1, ii = c / TL::GJ - 1;
-        const int gi = i0 + ii, gj = j0 + jj;
-        const bool ok = gi <= Nx && gj <= Ny;
-        const int col = ok ? wrap_p(gi, Nx - 1) * Ny + wrap_p(gj, Ny - 1) : 0;
-        cp_async<8>(t.ctopo + c, g.topo + col, ok);
-        cp_async<sizeof(R)>(t.cut_ + c, a.utau + col, ok);
-        cp_async<4>(t.cnzy + c, g.nzy + col, ok);
-        cp_async<4>(t.ccut + c, g.cut + col, ok);
-    }
-    for (int c = threadIdx.x; c < TL::GK * KROW; c += NT) {
-        const int gk = k0 - 1 + c / KROW;
-        const bool ok = gk >= 0 && gk < Nz;
-        cp_async<sizeof(R)>(t.kr + c, a.krow + (ok ? (size_t)gk * KROW + c % KROW : 0), ok);
-    }
-    if (!state) {
-        // the stage input arrives as a TMA box (see k_stage_fused)
-    } else if constexpr (TL::PAIRED && TL::SK * TL::SJ <= NT) {
-        // FP32 tile: thread (k, j) of the SK x SJ cross-section walks the SI
-        // planes in i, so the k/j arithmetic and the j wrap happen once per
-        // thread (lanes k fastest: global reads stay coalesced along k).  With
-        // twice the threads, two threads share a (k, j), half the planes each.
-        constexpr int KJ = TL::SK * TL::SJ, NSPLIT = (NT >= 2 * KJ && TL::SI % 2 == 0) ? 2 : 1;
-        if (threadIdx.x < KJ * NSPLIT) {
-            const int kj = threadIdx.x % KJ, part = threadIdx.x / KJ;
-            const int kk = kj % TL::SK - 2, jj = kj / TL::SK - 2;
-            const int gk = k0 + kk, gj = j0 + jj;
-            const bool okjk = gk >= 0 && gk < Nz && gj <= Ny + 1;
-            const size_t cj = okjk ? (size_t)wrap_p(gj, Ny - 1) * Nz + gk : 0;
-            const size_t plane = (size_t)Ny * Nz;
-            const int ii0 = -2 + part * (TL::SI / NSPLIT);
-#pragma unroll 2
-            for (int ii = ii0; ii < ii0 + TL::SI / NSPLIT; ii++) {
-                const int gi = i0 + ii;
-                const bool ok = okjk && gi <= Nx + 1;
-                const size_t o = ok ? (size_t)wrap_p(gi, Nx - 1) * plane + cj : 0;
-                const int sidx = TL::s(ii, jj, kk);
-#pragma unroll
-                for (int f = 0; f < 4; f++) cp_async<sizeof(R)>(t.st + TL::so(f, sidx), X + (size_t)f * N + o, ok);
-            }
-        }
-    } else {
-        for (int c = threadIdx.x; c < TL::SR; c += NT) {
-            const int kk = c % TL::SK - 2, jj = (c / TL::SK) % TL::SJ - 2, ii = c / (TL::SK * TL::SJ) - 2;
-            const int gk = k0 + kk;
-            const bool ok = gk >= 0 && gk < Nz && i0 + ii <= Nx + 1 && j0 + jj <= Ny + 1;
-            const size_t o = ok ? ((size_t)wrap_p(i0 + ii, Nx - 1) * Ny + wrap_p(j0 + jj, Ny - 1)) * Nz + gk : 0;
-#pragma unroll
-            for (int f = 0; f < 4; f++)
-                cp_async<sizeof(R)>(t.st + TL::so(f, TL::s(ii, jj, kk)), X + (size_t)f * N + o, ok);
-        }
-    }
-    cp_async_commit();
 }
 
 // Bounded wait on an mbarrier phase (false when the limit ran out).
@@ -196,659 +191,926 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int lim
     }
     return false;
 }
-constexpr int kTmaWaitLimit = 1 << 20;   // polls before a tile load is given up (about a second)
+constexpr int kTmaWaitLimit = 1 << 20;   // polls before a plane is given up (about a second)
 
-// FP32 tile from the TMA box: the box holds u, v, w, T (outermost) x SI x SJ
-// columns x 16 planes (k0-4 .. k0+11), one 64-byte row per column with the
-// 64-byte swizzle (16-byte chunk c of row r at chunk c ^ ((r >> 1) & 3)), so
-// the four chunk loads of consecutive columns hit distinct banks.  One thread
-// per (pair, column) writes the column's planes k0-2 .. k0+9 as (u, v) or
-// (w, T) pairs into the tile.
-template <class TL, int NT>
-__device__ __forceinline__ void repack_box(TL &t, const unsigned char *stg)
+// SGS inputs of a thread's cells
+template <class V> struct Sgs { V mu, g7, S11, S12, S13, S22, S23, S33; };
+template <class SM, class V> __device__ __forceinline__ void put_sgs(uint32_t o, const Sgs<V> &q)
 {
-    for (int c = threadIdx.x; c < 2 * TL::SI * TL::SJ; c += NT) {
-        const int jj = c % TL::SJ, r = c / TL::SJ, ii = r % TL::SI, pr = r / TL::SI;
-        const int ra = ((2 * pr) * TL::SI + ii) * TL::SJ + jj, rb = ra + TL::SI * TL::SJ;
-        float va[16], vb[16];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const float4 x = *reinterpret_cast<const float4 *>(stg + ra * 64 + ((q ^ ((ra >> 1) & 3)) << 4));
-            const float4 y = *reinterpret_cast<const float4 *>(stg + rb * 64 + ((q ^ ((rb >> 1) & 3)) << 4));
-            va[4 * q] = x.x; va[4 * q + 1] = x.y; va[4 * q + 2] = x.z; va[4 * q + 3] = x.w;
-            vb[4 * q] = y.x; vb[4 * q + 1] = y.y; vb[4 * q + 2] = y.z; vb[4 * q + 3] = y.w;
-        }
-        float2 *dst = reinterpret_cast<float2 *>(t.st) + pr * TL::SR + ii * TL::SK * TL::SJ + jj;
-#pragma unroll
-        for (int kk = 0; kk < TL::SK; kk++) dst[kk * TL::SJ] = make_float2(va[kk + 2], vb[kk + 2]);
+    sh<V>(o + G_MU * SM::FG) = q.mu;
+    sh<V>(o + G_Q * SM::FG) = q.g7;
+    sh<V>(o + G_S11 * SM::FG) = q.S11;
+    sh<V>(o + G_S12 * SM::FG) = q.S12;
+    sh<V>(o + G_S13 * SM::FG) = q.S13;
+    sh<V>(o + G_S22 * SM::FG) = q.S22;
+    sh<V>(o + G_S23 * SM::FG) = q.S23;
+    sh<V>(o + G_S33 * SM::FG) = q.S33;
+}
+
+// the z neighbours of the value at byte offset o (own value c): one plane below
+// and above, and two (FP32: the pair of cells k, k+1 takes k-2 .. k+3 from three
+// aligned pairs)
+template <class R, class V> struct ZNb { V m2, m1, p1, p2; };
+template <class R> __device__ __forceinline__ ZNb<R, typename Vec<R>::V> z_nb(uint32_t o, typename Vec<R>::V c)
+{
+    ZNb<R, typename Vec<R>::V> n;
+    if constexpr (sizeof(R) == 4) {
+        n.m2 = sh<F2>(o - 8);
+        n.p2 = sh<F2>(o + 8);
+        n.m1.v = make_float2(n.m2.v.y, c.v.x);
+        n.p1.v = make_float2(c.v.y, n.p2.v.x);
+    } else {
+        n.m2 = sh<double>(o - 16);
+        n.m1 = sh<double>(o - 8);
+        n.p1 = sh<double>(o + 8);
+        n.p2 = sh<double>(o + 16);
+    }
+    return n;
+}
+// difference of the planes above and below
+template <class R> __device__ __forceinline__ typename Vec<R>::V z_diff(uint32_t o, typename Vec<R>::V c)
+{
+    if constexpr (sizeof(R) == 4) {
+        const F2 p = {make_float2(c.v.y, sh<float>(o + 8))}, m = {make_float2(sh<float>(o - 4), c.v.x)};
+        return p - m;
+    } else {
+        return sh<double>(o + 8) - sh<double>(o - 8);
     }
 }
 
-// upwind derivative from 5 weights (zero weights leave the sum unchanged)
-template <class R> __device__ __forceinline__ R dz5(const R *w, R m2, R m1, R c, R p1, R p2)
-{
-    return w[0] * m2 + w[1] * m1 + w[2] * c + w[3] * p1 + w[4] * p2;
-}
+// Constants of the model as values of a thread's cells: a 64-bit constant is one
+// load, where a scalar would take two moves to fill a pair.
+template <class R> struct StageVec {
+    using V = typename Vec<R>::V;
+    V hx, hy, lx, ly, c12, c4, kT, inv_Trho_cp, H_C_cp, mu_Trho, Trho, two_inv_Trho, inv_Trho_Pr, g_Tinf, T_inf, third, m_third, half, p4, m_hx,
+        m_hy, ar, cA, cK;
+};
 
-// One RK stage over TI x TJ x KZ tiles (reference RHS pde.cu:139-787,
-// turbulence.cu:255-454, RK combination solver.cu:14-93).  One tile per block
-// (the grid is the tile count); two blocks per SM in FP32, so one block's tile
-// loads overlap the other's arithmetic.  Per tile:
-//   1. column tables, z rows, stage input with halo 2 -> shared memory
-//      (cp.async; the fuel fraction is read from global memory where needed)
-//   2. SGS inputs (raw mu_sgs, strain S', divergence source) on the tile and
-//      its halo 1 -> shared memory
-//   3. per tile cell: advection, diffusion, forces, reaction, SGS divergence,
-//      RK update.  Cells the boundary rules overwrite (k <= cut node, top) are
-//      left to k_stage_bc; the values it needs are stored in a.bc.
-template <class R, int TI, int TJ, int KZ, int NT>
-__global__ void __launch_bounds__(NT, sizeof(R) != 4 ? 1 : NT > 256 ? 2 : (TI * TJ <= 64 ? 3 : 2))
-    k_stage_fused(const StageArgs<R> a, const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap pyn,
-                  const __grid_constant__ CUtensorMap pacc, int use_tma, int use_pf, int ntk, int ntj, int nti)
+// Source terms of T and the divergence source g7 = nu T_RHS / T of the SGS model
+// (pde.cu:640-760): conduction and radiation over rho c_p, reaction, and unless
+// LEAN the Sutherland laws and the convective exchange.  1 / rho is
+// T / (T_inf rho_inf); x^(3/2) and x^(1/4) are taken by square roots.
+template <class R, class V, bool LEAN>
+__device__ __forceinline__ void sources(const StageArgs<R> &a, const StageVec<R> &q, V Tx, V Ty, V Tz, V lapT, V T, V Y, V K_T, int gk,
+                                        int nzy, V dz, V &src, V &nu, V &g7)
 {
-    using TL = Tile<R, TI, TJ, KZ>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    R *sgs = reinterpret_cast<R *>(smem_raw + TL::BUF);
-    R *s_vd = reinterpret_cast<R *>(smem_raw + TL::O_MISC);
-    int *s_fail = reinterpret_cast<int *>(smem_raw + TL::O_MISC + 8);
-    int *s_vd_zero = reinterpret_cast<int *>(smem_raw + TL::O_MISC + 12);
-    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(smem_raw + TL::O_MISC + 16);
-    const Geom &g = a.g;
-    const PhysR<R> &p = a.pr;
-    const int Nx = g.Nx, Ny = g.Ny, Nz = g.Nz, N = g.N;
-    const R *__restrict__ X = a.X;
-    const int ntiles = ntk * ntj * nti;
-    const int tile = blockIdx.x;   // one tile per block
-    if (tile >= ntiles) return;
-    {
-        TL t;
-        t.bind(smem_raw, sgs);
-        const int k0 = (tile % ntk) * KZ, j0 = ((tile / ntk) % ntj) * TJ, i0 = (tile / (ntk * ntj)) * TI;
-        // FP32 tiles whose halo stays inside the stored planes 0..N-2 (no periodic
-        // wrap) arrive as one TMA box of u, v, w, T; the others by cp.async
-        bool tma = false;
-        if constexpr (TL::PAIRED)
-            tma = use_tma && i0 >= 2 && i0 + TI + 1 <= Nx - 2 && j0 >= 2 && j0 + TJ + 1 <= Ny - 2 &&
-                  (((uint32_t)__cvta_generic_to_shared(sgs)) & 511u) == 0;
-        if (threadIdx.x == 0) {
-            *s_fail = 0;
-            if (tma) {
-                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-                asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    const V T2 = T * T, gg = vfma(Tz, Tz, vfma(Ty, Ty, Tx * Tx));
+    V mu_Trho = q.mu_Trho, kT = q.kT, dk = splat<V>(R(0)), ex = dk, ext = dk;
+    if constexpr (!LEAN) {
+        const PhysR<R> &p = a.pr;
+        auto c = [](double x) { return splat<V>((R)x); };
+        if (a.ph.sutherland_viscosity == 1 || a.ph.sutherland_conductivity == 1) {
+            const V x = T * c(1.0 / 273.15), sx = vsqrt(x), x15 = x * sx;
+            if (a.ph.sutherland_viscosity == 1)
+                mu_Trho = vdiv(x15 * c(1.716e-5 * (273.15 + 110.4)), (T + c(110.4)) * splat<V>(p.Trho));
+            if (a.ph.sutherland_conductivity == 1) {
+                const V d = vdiv(c(0.0241 * (273.15 + 194)), T + c(194));
+                kT = d * x15;
+                dk = d * vfma(c(1.5), sx, vdiv(c(-1.0) * x15, T + c(194)));
             }
         }
-        __syncthreads();   // barrier initialised before anyone waits on it
-        if (tma && threadIdx.x == 0) {
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)TL::BOX)
-                         : "memory");
+        if (p.alpha_s * p.sigma_s != R(0)) {
+            // the gas is at T where the cell holds no fuel, the solid where it does; the other
+            // of the two, and both above the fuel zone, at T_inf
+            V dT, Tg;
+#pragma unroll
+            for (int e = 0; e < Vec<R>::W; e++) {
+                const bool solid = el(Y, e) > R(0);
+                set_el(Tg, e, solid ? p.T_inf : el(T, e));
+                set_el(dT, e, gk + e > nzy ? R(0) : solid ? p.T_inf - el(T, e) : el(T, e) - p.T_inf);
+            }
+            V ad;
+#pragma unroll
+            for (int e = 0; e < Vec<R>::W; e++) set_el(ad, e, rfabs(el(dT, e)));
+            const V h = splat<V>(p.h_c) * dz * vsqrt(vsqrt(vdiv(ad, dz)));
+            ex = h * splat<V>(-p.alpha_s * p.sigma_s) * dT;
+            ext = Tg * q.inv_Trho_cp;
+        }
+    }
+    const V cond = vfma(q.c4, T2 * T, kT);
+    const V flux = LEAN ? q.c12 * T2 * gg : vfma(q.c12 * T2, gg, dk);
+    src = vfma(cond, lapT, flux) * (T * q.inv_Trho_cp);
+    src = vfma(q.H_C_cp * Y, K_T, src);
+    if constexpr (!LEAN) src = vfma(ex, ext, src);
+    nu = mu_Trho * T;
+    g7 = mu_Trho * src;
+}
+
+// differences of one field across a cell, over two spacings
+template <class V> struct Grad { V x, y, z; };
+
+// Squared Van Driest factors (turbulence.cu:255-454) of points at heights zh in a
+// column of terrain height topo and friction velocity ut, with q = -1 / (A nu) of
+// the cells they are taken for.
+template <class R, class V> __device__ __forceinline__ V vd_factor2(V zh, R topo, R ut, V q)
+{
+    V f = vpos(zh - splat<V>(topo)) * splat<V>(ut) * q;
+#pragma unroll
+    for (int e = 0; e < Vec<R>::W; e++) set_el(f, e, van_driest(el(f, e)));
+    return f * f;
+}
+__device__ __forceinline__ F2 vshfl(F2 a, int l)
+{
+    return {make_float2(__shfl_sync(0xffffffffu, a.v.x, l), __shfl_sync(0xffffffffu, a.v.y, l))};
+}
+__device__ __forceinline__ double vshfl(double a, int l) { return __shfl_sync(0xffffffffu, a, l); }
+
+// SGS inputs from the differences (pde.cu:632-765): traceless strain S_ii = d_i u_i
+// - div / 3, mu_sgs = rho l2 |S|.  Every sum of products is an explicit fused
+// multiply-add, here and wherever the frame and the tile evaluate the same value:
+// left to the compiler, the two came out differently in the last bit.
+template <class R, class V> __device__ __forceinline__ Sgs<V> strain(const StageVec<R> &c, const Grad<V> (&d)[4], V hz, V T, V l2, V g7)
+{
+    Sgs<V> q;
+    const V ux = d[0].x * c.hx, vy = d[1].y * c.hy, wz = d[2].z * hz;
+    const V s12 = vfma(d[0].y, c.hy, d[1].x * c.hx), s13 = vfma(d[0].z, hz, d[2].x * c.hx), s23 = vfma(d[2].y, c.hy, d[1].z * hz);
+    const V sq = vfma(wz, wz, vfma(vy, vy, ux * ux));
+    const V mod2 = vfma(s23, s23, vfma(s12, s12, vfma(s13, s13, sq + sq)));
+    const V div = vfma(d[2].z, hz, vfma(d[1].y, c.hy, ux));
+    q.S11 = vfma(div, c.m_third, ux);
+    q.S22 = vfma(div, c.m_third, vy);
+    q.S33 = vfma(div, c.m_third, wz);
+    q.S12 = c.half * s12;
+    q.S13 = c.half * s13;
+    q.S23 = c.half * s23;
+    q.mu = vdiv(c.Trho * l2, T) * vsqrt(mod2);
+    q.g7 = g7;
+    return q;
+}
+
+template <class R, int NT, int FR, int NB, int KW, bool LEAN, bool VEC>
+__global__ void __launch_bounds__(NT + FR, NB)
+    k_stage_march(const StageArgs<R> a, const StageVec<R> cv, const StageGrid sg, const __grid_constant__ CUtensorMap m_tile,
+                  const __grid_constant__ CUtensorMap m_row)
+{
+    using SM = StageSmem<R, KW>;
+    using V = typename Vec<R>::V;
+    constexpr int VW = Vec<R>::W;
+    constexpr uint32_t E = sizeof(R);
+    const Geom &g = a.g;
+    const PhysR<R> &p = a.pr;
+    const int Nx = g.Nx, Ny = g.Ny, Nz = g.Nz;
+    const int tj = sg.tj, tk = sg.tk;
+    const SM sm(tj);
+    int bid = blockIdx.x;
+    const int k0 = (bid % sg.ntk) * tk;
+    bid /= sg.ntk;
+    const int j0 = (bid % sg.ntj) * tj, ib = (bid / sg.ntj) * sg.L;
+    const int ie = min(ib + sg.L, Nx);
+    const int tid = threadIdx.x;
+    const bool tma = sg.tma;
+    // offsets within one field are below 4 GiB (wf_create's limit on the grid), so
+    // addresses are a uniform base per field and a 32-bit byte offset
+    const uint32_t plane = (uint32_t)Ny * (uint32_t)Nz * E;
+    const size_t FB = (size_t)g.N * E;
+    const int CW = tj + 2;
+    auto at = [&](const R *base, int f, uint32_t o) -> const R & {
+        return *reinterpret_cast<const R *>(reinterpret_cast<const char *>(base) + f * FB + o);
+    };
+    auto c_ = [](R x) { return splat<V>(x); };
+    const bool rd = stage_reads_acc(a.method, a.stage), kp = stage_keeps_acc(a.method, a.stage), kstore = a.method == 3;
+
+    // z weights of the tile's planes and the walls' one-sided weights
+    for (int c = tid; c < SM::PG * ZROW; c += NT + FR) {
+        const int e = c / SM::PG, kk = c - e * SM::PG, gk = k0 - 2 + kk;
+        R v = R(0);
+        if (gk >= 0 && gk < Nz) {
+            const R *r = a.krow + (size_t)gk * KROW;
+            const bool wall = gk == 0 || gk == Nz - 1;
+            if (e < ZF) v = (gk >= 2) ? -r[RKM + e] : R(0);
+            else if (e < ZWP) v = (gk <= Nz - 3) ? -r[RKP + 2 + e - ZF] : R(0);
+            else if (e == ZWP) v = (gk == 1 || gk == Nz - 2) ? R(0) : R(1);
+            else if (e == ZWW) v = gk == Nz - 2 ? R(1) : R(0);
+            else if (e == ZD1) v = wall ? a.krow[(gk == 0 ? 1 : Nz - 2) * KROW + RD1] : r[RD1];
+            else if (e == ZL) v = a.coef ? r[RDD2] : r[RDEL2];
+            else if (e < ZZ) v = r[RD2 + 2 * (e - ZD2)];
+            else v = e == ZZ ? r[RZ] : r[RDZ];
+        }
+        if (e == ZDZ && v == R(0)) v = R(1);   // outside the grid: a divisor
+        sh<R>(sm.zr + c * E) = v;
+    }
+    // The one-sided first derivative on a wall (pde.cu:363-576) as the centred one
+    // with a value beyond the wall, f1 - D / w (w the centred weight): weights of
+    // that value; and the one-sided second derivative of T
+    if (tid < 14) {
+        const double *zc = g.zc;
+        const int q = tid % 7, top = Nz - 1;
+        const bool bot = tid < 7;
+        const double w = bot ? zc[ZC * Nz + 1] : zc[ZC * Nz + top - 1];
+        double v;
+        if (q < 3) {
+            v = bot ? -zc[(ZF0 + q) * Nz] / w : zc[(ZB2 - q) * Nz + top] / w;
+            if (q == 1) v += 1.0;
+        } else {
+            v = bot ? zc[(ZFF0 + q - 3) * Nz] : zc[(ZBB3 - (q - 3)) * Nz + top];
+        }
+        sh<R>(sm.wall + tid * E) = (R)v;
+    }
+    if (tid < VW) sh<R>(sm.corr + (4 * CW * VW + tid) * E) = R(0);
+
+    auto block_sync = [&]() { asm volatile("bar.sync 0, %0;" ::"n"(NT + FR) : "memory"); };
+    auto up = [](int r, int d, int n) { return r + d >= n ? r + d - n : r + d; };   // ring slot d planes on
+    auto col_slot = [&](int c) { return (uint32_t)((c & (kColRing - 1)) * CW); };
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(stage_smem);
+
+    // ---- state planes into the ring ----
+    if (tma && tid == 0) {
+        for (int r = 0; r < SM::RS; r++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sbase + sm.bar + r * 8) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (tma) block_sync();
+    // by TMA, issued by one lane of the block's last warp: a box of the tile's rows,
+    // or one per row where the tile's halo wraps around in y
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // uniform in a warp
+    const bool issuer = warp == (NT + FR) / 32 - 1 && (tid & 31) == 0;
+    const bool wraps = j0 < 2 || j0 + tj + 1 > Ny - 2;
+    auto fetch_box = [&](int c, int slot) {
+        if (!issuer) return;
+        const uint32_t bar = sbase + sm.bar + slot * 8, dst = sbase + slot * sm.planeS;
+        const int ci = wrap_p(c, Nx - 1);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)(tj + 4) * SM::ROW_S) : "memory");
+        const uint64_t map = reinterpret_cast<uint64_t>(wraps ? &m_row : &m_tile);
+        const int n = wraps ? tj + 4 : 1;
+#pragma unroll 1
+        for (int r = 0; r < n; r++)
             asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
                          "[%0], [%1, {%2, %3, %4, %5}], [%6];"
                          :
-                         : "r"((uint32_t)__cvta_generic_to_shared(sgs)), "l"(reinterpret_cast<uint64_t>(&tmap)),
-                           "r"(k0 - 4), "r"(j0 - 2), "r"(i0 - 2), "r"(0), "r"(bar)
+                         : "r"(dst + r * SM::ROW_S), "l"(map), "r"(k0 - SM::KH), "r"(0), "r"(wrap_p(j0 - 2 + r, Ny - 1)), "r"(ci), "r"(bar)
                          : "memory");
+    };
+    // the RK operands of x-plane c of the tile into L2: frame threads, a row of one
+    // field each
+    auto prefetch_rk = [&](int c) {
+        for (int q = tid - NT; q < 8 * tj; q += FR) {
+            const int f = q & 3, row = q >> 3;
+            const bool acc = q & 4;
+            if (j0 + row < Ny && (acc ? rd : !kstore))
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(
+                    &at(acc ? a.acc : a.yn, f, (uint32_t)c * plane + ((uint32_t)(j0 + row) * (uint32_t)Nz + k0) * E)));
         }
-        // RK operands of the tile's cells (yn, and acc when this stage reads it)
-        // into L2 while the tile loads and phase 2 runs: phase 3 then finds
-        // them there instead of waiting on DRAM.  A prefetch has no completion
-        // to wait for and ignores coordinates outside the buffer.
-        if (use_pf && threadIdx.x == 32) {
-            asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];"
-                         :
-                         : "l"(reinterpret_cast<uint64_t>(&pyn)), "r"(k0), "r"(j0), "r"(i0), "r"(0)
-                         : "memory");
-            if (stage_reads_acc(a.method, a.stage))
-                asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];"
-                             :
-                             : "l"(reinterpret_cast<uint64_t>(&pacc)), "r"(k0), "r"(j0), "r"(i0), "r"(0)
-                             : "memory");
+    };
+    // column tables of x-plane c, row jj: loaded, and put into the ring
+    struct Col {
+        double topo;
+        R ut;
+        int2 ix;
+    };
+    auto get_col = [&](int c, int jj) {
+        Col q = {0.0, R(0), make_int2(0, 0)};
+        if (j0 + jj <= Ny) {
+            const int col = wrap_p(c, Nx - 1) * Ny + wrap_p(j0 + jj, Ny - 1);
+            q.topo = g.topo[col];
+            q.ut = a.utau[col];
+            q.ix = make_int2(g.nzy[col], g.cut[col]);
         }
-        issue_tile<R, TL, NT>(a, t, i0, j0, k0, !tma);
-        cp_async_wait<0>();
-        if (tma) {
-            if (!mbar_wait(bar, 0, kTmaWaitLimit)) *s_fail = 1;
-            else repack_box<TL, NT>(t, reinterpret_cast<const unsigned char *>(sgs));
-        }
-        __syncthreads();
-        if (*s_fail) {
-            // the box did not arrive in time: flag it, give the copy a bounded
-            // chance to land (it writes this block's shared memory), leave the tile
-            if (threadIdx.x == 0) {
-                if (a.kerr) atomicExch(a.kerr, 1);
-                mbar_wait(bar, 0, kTmaWaitLimit);
-            }
-            __syncthreads();
-            return;
-        }
+        return q;
+    };
+    auto put_col = [&](int c, int jj, const Col &q) {
+        const uint32_t o = col_slot(c) + jj + 1;
+        sh<R>(sm.ctopo + o * E) = (R)q.topo;
+        sh<R>(sm.cut_ + o * E) = q.ut;
+        sh<int2>(sm.cidx + o * 8) = q.ix;
+    };
 
-        const int smu = a.ph.sutherland_viscosity, sk = a.ph.sutherland_conductivity;
-        // FP32 path without Sutherland laws or convective exchange: the
-        // divergence source nu T_RHS / T reduces to mu/(T_inf rho_inf) T_RHS
-        const bool lean = sizeof(R) == 4 && smu != 1 && sk != 1 && !(p.alpha_s * p.sigma_s != R(0));
-
-        // Lower bound over the tile of z_ibm u_tau / A_vd, taken over the
-        // columns with wall friction: when it exceeds the cut-off times nu,
-        // every Van Driest factor of those columns is exactly 1, and every
-        // factor of a column without friction (u_tau = 0, as over the hills)
-        // is 1 - exp(-0) = 0 at any height.
-        R &s_vd_bound = *s_vd;
-        if (threadIdx.x < 32) {
-            const R zlow = (k0 > 0) ? t.K(-1, RZ) : R(0);
-            R hmax = R(-1e30), umin = R(1e30);
-            bool zero = false;
-            for (int c = threadIdx.x; c < TL::NCOL; c += 32) {
-                const R ut = t.cut_[c];
-                if (ut == R(0)) {
-                    zero = true;
-                } else {
-                    hmax = rmax(hmax, (R)t.ctopo[c]);
-                    umin = rmin(umin, ut);
-                }
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                hmax = rmax(hmax, __shfl_xor_sync(0xffffffffu, hmax, o));
-                umin = rmin(umin, __shfl_xor_sync(0xffffffffu, umin, o));
-            }
-            zero = __any_sync(0xffffffffu, zero);
-            if (threadIdx.x == 0) {
-                s_vd_bound = rmax(zlow - hmax, R(0)) * rmax(umin, R(0)) * p.inv_avd;
-                *s_vd_zero = zero;
-            }
+    // ---- this thread's cells: of the tile (tid < NT), or of the frame ----
+    const bool frame = warp >= NT / 32;
+    const int h = tid - NT;   // frame thread
+    int jj, kk;
+    bool in;
+    if (!frame) {
+        const int w = tk / VW;
+        jj = tid / w;
+        kk = (tid - jj * w) * VW;
+        in = jj < tj;
+    } else {
+        // rows above and below the tile, then the planes above and below it (FP32:
+        // the pair that holds the plane)
+        const int w = tk / VW;
+        in = h < 2 * w + 2 * tj;
+        if (h < 2 * w) {
+            jj = h < w ? -1 : tj;
+            kk = (h < w ? h : h - w) * VW;
+        } else {
+            const int e = h - 2 * w;
+            jj = e < tj ? e : e - tj;
+            kk = e < tj ? -VW : tk;
         }
-
-        // ---- 2. SGS inputs on the tile and its halo 1 (pde.cu:632-765).  Needed
-        //        set: tile columns on k0-1 .. k0+KZ, side columns on k0 .. k0+KZ-1.
-        //        Enumerated so that each warp covers 8 consecutive k x 4 j where
-        //        it can: tile columns k0-1..k0+6, tile columns k0+7..k0+8,
-        //        x-side columns, y-side columns.
-        //        In the 8-plane groups the lanes of a warp are 4 j (fastest) x 8 k.
-        static_assert(KZ == 8 && TJ % 4 == 0 && NT % 32 == 0, "phase-2/3 enumeration: 8 planes, 4-column lane groups");
-        constexpr int NA1 = TI * TJ * 8, NA2 = TI * TJ * 2, NB = 2 * TJ * KZ, NC = TI * 2 * KZ;
-        static_assert(NA1 % 32 == 0 && NA2 % 32 == 0, "warp-aligned groups");
-        for (int c = threadIdx.x; c < NA1 + NA2 + NB + NC; c += NT) {
-            int ii, jj, kk;
-            if (c < NA1) {
-                kk = ((c & 31) >> 2) - 1;
-                jj = ((c >> 5) % (TJ / 4)) * 4 + (c & 3);
-                ii = (c >> 5) / (TJ / 4);
-            } else if (c < NA1 + NA2) {
-                const int d = c - NA1;
-                jj = d % TJ;
-                kk = 7 + (d / TJ) % 2;
-                ii = d / (2 * TJ);
-            } else if (c < NA1 + NA2 + NB) {
-                const int d = c - NA1 - NA2;
-                kk = (d & 31) >> 2;
-                jj = ((d >> 5) % (TJ / 4)) * 4 + (d & 3);
-                ii = ((d >> 5) / (TJ / 4)) ? TI : -1;
-            } else {
-                const int d = c - NA1 - NA2 - NB;
-                kk = d % KZ;
-                jj = ((d / KZ) % 2) ? TJ : -1;
-                ii = d / (2 * KZ);
-            }
-            const int gk = k0 + kk;
-            if (gk < 0 || gk >= Nz || i0 + ii > Nx || j0 + jj > Ny) continue;
-            R ux, uy, uz, vx, vy, vz, wx, wy, wz, Tc, Tx, Ty, Tz, Txx, Tyy, Tzz;
-            bool zdone = false;
-            if constexpr (TL::PAIRED) {
-                const float2 UVxp = t.P(0, ii + 1, jj, kk), UVxm = t.P(0, ii - 1, jj, kk);
-                const float2 UVyp = t.P(0, ii, jj + 1, kk), UVym = t.P(0, ii, jj - 1, kk);
-                const float2 WTxp = t.P(1, ii + 1, jj, kk), WTxm = t.P(1, ii - 1, jj, kk);
-                const float2 WTyp = t.P(1, ii, jj + 1, kk), WTym = t.P(1, ii, jj - 1, kk);
-                const float2 i2x = bcast(p.inv2dx), i2y = bcast(p.inv2dy);
-                const float2 dUVx = mul2(sub2(UVxp, UVxm), i2x), dUVy = mul2(sub2(UVyp, UVym), i2y);
-                const float2 dWTx = mul2(sub2(WTxp, WTxm), i2x), dWTy = mul2(sub2(WTyp, WTym), i2y);
-                ux = dUVx.x; vx = dUVx.y; wx = dWTx.x; Tx = dWTx.y;
-                uy = dUVy.x; vy = dUVy.y; wy = dWTy.x; Ty = dWTy.y;
-                Tc = t.P(1, ii, jj, kk).y;
-                Txx = (WTxp.y - R(2) * Tc + WTxm.y) * p.invdx2;
-                Tyy = (WTyp.y - R(2) * Tc + WTym.y) * p.invdy2;
-                if (gk > 0 && gk < Nz - 1) {
-                    const float2 UVzp = t.P(0, ii, jj, kk + 1), UVzm = t.P(0, ii, jj, kk - 1);
-                    const float2 WTzp = t.P(1, ii, jj, kk + 1), WTzm = t.P(1, ii, jj, kk - 1);
-                    const float2 wc = bcast(t.K(kk, RD1));
-                    const float2 dUVz = mul2(sub2(UVzp, UVzm), wc), dWTz = mul2(sub2(WTzp, WTzm), wc);
-                    uz = dUVz.x; vz = dUVz.y; wz = dWTz.x; Tz = dWTz.y;
-                    Tzz = t.K(kk, RD2) * WTzm.y + t.K(kk, RD2 + 1) * Tc + t.K(kk, RD2 + 2) * WTzp.y;
-                    zdone = true;
-                }
-            } else {
-                Tc = t.S(3, ii, jj, kk);
-                ux = (t.S(0, ii + 1, jj, kk) - t.S(0, ii - 1, jj, kk)) * p.inv2dx;
-                uy = (t.S(0, ii, jj + 1, kk) - t.S(0, ii, jj - 1, kk)) * p.inv2dy;
-                vx = (t.S(1, ii + 1, jj, kk) - t.S(1, ii - 1, jj, kk)) * p.inv2dx;
-                vy = (t.S(1, ii, jj + 1, kk) - t.S(1, ii, jj - 1, kk)) * p.inv2dy;
-                wx = (t.S(2, ii + 1, jj, kk) - t.S(2, ii - 1, jj, kk)) * p.inv2dx;
-                wy = (t.S(2, ii, jj + 1, kk) - t.S(2, ii, jj - 1, kk)) * p.inv2dy;
-                const R Txp = t.S(3, ii + 1, jj, kk), Txm = t.S(3, ii - 1, jj, kk);
-                const R Typ = t.S(3, ii, jj + 1, kk), Tym = t.S(3, ii, jj - 1, kk);
-                Tx = (Txp - Txm) * p.inv2dx;
-                Ty = (Typ - Tym) * p.inv2dy;
-                Txx = (Txp - R(2) * Tc + Txm) * p.invdx2;
-                Tyy = (Typ - R(2) * Tc + Tym) * p.invdy2;
-                if (gk > 0 && gk < Nz - 1) {
-                    const R wc = t.K(kk, RD1);
-                    uz = (t.S(0, ii, jj, kk + 1) - t.S(0, ii, jj, kk - 1)) * wc;
-                    vz = (t.S(1, ii, jj, kk + 1) - t.S(1, ii, jj, kk - 1)) * wc;
-                    wz = (t.S(2, ii, jj, kk + 1) - t.S(2, ii, jj, kk - 1)) * wc;
-                    Tz = (t.S(3, ii, jj, kk + 1) - t.S(3, ii, jj, kk - 1)) * wc;
-                    Tzz = t.K(kk, RD2) * t.S(3, ii, jj, kk - 1) + t.K(kk, RD2 + 1) * Tc + t.K(kk, RD2 + 2) * t.S(3, ii, jj, kk + 1);
-                    zdone = true;
-                }
-            }
-            if (!zdone) {
-                // walls: one-sided stencils from the double table (planes k = 0 and Nz-1 only)
-                const double *zc = g.zc;
-                const bool bot = (gk == 0);
-                auto d1 = [&](int f) -> R {
-                    if (bot)
-                        return (R)zc[ZF0 * Nz] * t.S(f, ii, jj, kk) + (R)zc[ZF1 * Nz] * t.S(f, ii, jj, kk + 1) +
-                               (R)zc[ZF2 * Nz] * t.S(f, ii, jj, kk + 2);
-                    return (R)zc[ZB0 * Nz + gk] * t.S(f, ii, jj, kk - 2) + (R)zc[ZB1 * Nz + gk] * t.S(f, ii, jj, kk - 1) +
-                           (R)zc[ZB2 * Nz + gk] * t.S(f, ii, jj, kk);
-                };
-                uz = d1(0);
-                vz = d1(1);
-                wz = d1(2);
-                Tz = d1(3);
-                // the backward 4-point form needs k-3, inside the tile unless the
-                // top plane is alone in its tile (then no cell of this tile needs it)
-                const R m3 = (kk >= 1) ? t.S(3, ii, jj, kk - 3) : R(0), p3 = (kk <= KZ - 2) ? t.S(3, ii, jj, kk + 3) : R(0);
-                Tzz = bot ? (R)zc[ZFF0 * Nz] * Tc + (R)zc[ZFF1 * Nz] * t.S(3, ii, jj, kk + 1) +
-                                (R)zc[ZFF2 * Nz] * t.S(3, ii, jj, kk + 2) + (R)zc[ZFF3 * Nz] * p3
-                          : (R)zc[ZBB0 * Nz + gk] * m3 + (R)zc[ZBB1 * Nz + gk] * t.S(3, ii, jj, kk - 2) +
-                                (R)zc[ZBB2 * Nz + gk] * t.S(3, ii, jj, kk - 1) + (R)zc[ZBB3 * Nz + gk] * Tc;
-            }
-            const R rho = fdiv(p.Trho, Tc);
-            const R S11 = third(R(2) * ux) - third(vy + wz);
-            const R S22 = third(R(2) * vy) - third(ux + wz);
-            const R S33 = third(R(2) * wz) - third(ux + vy);
-            const R mod_S = rsqrt_(R(2) * (ux * ux + vy * vy + wz * wz) + (uz + wx) * (uz + wx) + (vx + uy) * (vx + uy) +
-                                   (wy + vz) * (wy + vz));
-            const int nzy = t.cnzy[TL::cq(ii, jj)];
-            // fuel fraction of the stage input (used only below the column's fuel top)
-            const R Yq = (gk < nzy) ? X[4 * (size_t)N + (size_t)(wrap_p(i0 + ii, Nx - 1) * Ny + wrap_p(j0 + jj, Ny - 1)) * g.NzY + gk]
-                                    : R(0);
-            R g7;
-            if (lean) {
-                const R K_T = arrhenius(p, Tc);
-                const R Yv = (gk < nzy) ? Yq : R(0);
-                const R T2 = Tc * Tc;
-                g7 = p.mu_Trho * ((p.c12 * T2 * (Tx * Tx + Ty * Ty + Tz * Tz) + (p.kT + p.c4 * (T2 * Tc)) * (Txx + Tyy + Tzz)) *
-                                      (Tc * p.inv_Trho_cp) +
-                                  p.H_C_cp * Yv * K_T);
-            } else {
-                const Thermo<R> th = thermo(p, smu, sk, Tc, t.S(3, ii, jj, kk + 1), Yq, gk, nzy, Tx, Ty, Tz,
-                                            Txx + Tyy + Tzz, t.K(kk, RDZ), rho);
-                g7 = fdiv(th.nu * th.T_RHS_tmp, Tc);
-            }
-            if (a.coef) {
-                // learned closure: the coefficient of this point replaces C_s^2
-                const R cq = a.coef[((size_t)wrap_p(i0 + ii, Nx - 1) * Ny + wrap_p(j0 + jj, Ny - 1)) * Nz + gk];
-                t.G(0, ii, jj, kk) = rho * (t.K(kk, RDD2) * cq) * mod_S;
-            } else {
-                t.G(0, ii, jj, kk) = rho * t.K(kk, RDEL2) * mod_S;
-            }
-            t.G(1, ii, jj, kk) = S11;
-            t.G(2, ii, jj, kk) = R(0.5) * (uy + vx);
-            t.G(3, ii, jj, kk) = R(0.5) * (uz + wx);
-            t.G(4, ii, jj, kk) = S22;
-            t.G(5, ii, jj, kk) = R(0.5) * (wy + vz);
-            t.G(6, ii, jj, kk) = S33;
-            t.G(7, ii, jj, kk) = g7;
-        }
-        __syncthreads();
-
-        // ---- 3. right-hand side, SGS divergence, RK update per tile cell
-        const R an = (R)a.a_next;
-        const bool rd = stage_reads_acc(a.method, a.stage), kp = stage_keeps_acc(a.method, a.stage);
-        for (int c = threadIdx.x; c < TL::CELLS; c += NT) {
-            // lanes: 4 j (fastest) x 8 k, as in phase 2
-            const int kk = (c & 31) >> 2, jj = ((c >> 5) % (TJ / 4)) * 4 + (c & 3), ii = (c >> 5) / (TJ / 4);
-            const int gi = i0 + ii, gj = j0 + jj, gk = k0 + kk;
-            if (gi >= Nx || gj >= Ny || gk >= Nz) continue;
-            const int col = gi * Ny + gj;
-            const int cc = TL::cq(ii, jj);
-            const int kc = t.ccut[cc], nzy = t.cnzy[cc];
-            const size_t cg = (size_t)col * Nz + gk;
-            if (gk < kc) {
-                // dead node below the terrain: the boundary rules fix its k-values (pde.cu:88-97)
-                const double dv[4] = {a.ph.u_dead, a.ph.v_dead, a.ph.w_dead, a.ph.T_dead};
+    }
+    if (!in) jj = kk = 0;
+    const int gj = j0 + jj, gk = k0 + kk;
+    const bool comp = in && gj <= Ny && gk < Nz && gk + VW > 0;   // SGS inputs wanted
+    const bool fuelz = comp && gk < g.NzY;                        // may hold fuel
+    const uint32_t so = SM::s(jj, kk), go = sm.g0 + SM::g(jj, kk), zo = sm.zr + SM::z(kk);
+    const uint32_t off = comp ? ((uint32_t)wrap_p(gj, Ny - 1) * (uint32_t)Nz + (uint32_t)max(gk, 0)) * E : 0;
+    // second z derivative of T of a wall cell (others: the zero)
+    const int side = gk <= 0 ? 0 : gk + VW >= Nz ? 1 : 2;
+    const uint32_t co = sm.corr + (side == 2 || !comp ? 4 * CW : side * CW + jj + 1) * (VW * E), cstep = side == 2 || !comp ? 0 : 2 * CW * VW * E;
+    // fuel fraction and learned coefficient of the stage input at x-plane c
+    auto fuel_at = [&](int c) -> V {
+        V Y = c_(R(0));
+        if (fuelz) {
+            const int nzy = sh<int2>(sm.cidx + (col_slot(c) + jj + 1) * 8).x;
+            const uint32_t o = (uint32_t)(wrap_p(c, Nx - 1) * Ny + wrap_p(gj, Ny - 1)) * (uint32_t)g.NzY;
 #pragma unroll
-                for (int f = 0; f < 4; f++) rk_cell(a, (size_t)f * N + cg, (R)dv[f], rd, kp, an);
-                if (gk < g.NzY)
-                    rk_cell(a, 4 * (size_t)N + (size_t)col * g.NzY + gk, (gk < nzy) ? (R)a.ph.Y_dead : R(0), rd, kp, an);
-                continue;
+            for (int e = 0; e < VW; e++)
+                if (gk + e >= 0 && gk + e < nzy) set_el(Y, e, at(a.X, 4, (o + gk + e) * E));
+        }
+        return Y;
+    };
+    auto coef_at = [&](int c) -> V {
+        V q = c_(R(1));
+        if (a.coef && comp) {
+#pragma unroll
+            for (int e = 0; e < VW; e++)
+                if (gk + e >= 0 && gk + e < Nz)
+                    set_el(q, e, a.coef[((size_t)wrap_p(c, Nx - 1) * Ny + wrap_p(gj, Ny - 1)) * Nz + gk + e]);
+        }
+        return q;
+    };
+    auto arrhenius_v = [&](V T) {
+        V K = c_(R(0));
+        if (fuelz)
+#pragma unroll
+            for (int e = 0; e < VW; e++) set_el(K, e, arrhenius(p, el(T, e)));
+        return K;
+    };
+
+    // by cp.async: every thread its own cells, and of the frame the rows two away (the
+    // planes two away are in its pairs) or a corner; zeros outside the grid
+    int j2 = jj;
+    if (frame && in) j2 = jj < 0 ? -2 : jj == tj ? tj + 1 : jj == 0 ? -1 : jj == tj - 1 ? tj : jj;
+    auto copy_cells = [&](int c, int slot, int row) {
+        const int gr = j0 + row;
+        const uint32_t ci = (uint32_t)wrap_p(c, Nx - 1) * plane + ((uint32_t)wrap_p(gr, Ny - 1) * (uint32_t)Nz + gk) * E;
+        // FP64: a frame thread of the planes next to the tile also takes those two away
+        const int e0 = VW == 1 && frame && kk < 0 ? -1 : 0, e1 = VW == 1 && frame && kk == tk ? 2 : VW;
+#pragma unroll
+        for (int e = -1; e < 2; e++) {
+            if (e < e0 || e >= e1) continue;
+            const bool ok = gk + e >= 0 && gk + e < Nz && gr <= Ny + 1;
+            const uint32_t d = slot * sm.planeS + SM::s(row, kk + e);
+#pragma unroll
+            for (int f = 0; f < 4; f++) cp_async<E>(d + f * SM::FX, &at(a.X, f, ok ? ci + e * E : 0), ok);
+        }
+    };
+    auto fetch_copy = [&](int c, int slot) {
+        if (in) {
+            copy_cells(c, slot, jj);
+            if (j2 != jj) copy_cells(c, slot, j2);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int lost = -1;   // slot whose plane did not arrive in time: flagged, no further fetches and waits
+    auto fetch = [&](int c, int slot) {
+        if (!tma) fetch_copy(c, slot);
+        else if (lost < 0) fetch_box(c, slot);
+    };
+    uint32_t phases = 0;
+    auto arrived = [&](int slot) {
+        if (tma && lost < 0) {
+            if (mbar_wait(sbase + sm.bar + slot * 8, (phases >> slot) & 1, kTmaWaitLimit)) {
+                phases ^= 1u << slot;
+            } else {
+                lost = slot;
+                if (a.kerr) atomicExch(a.kerr, 1);
             }
-            const bool live = (gk > kc) && (gk < Nz - 1);                 // not overwritten by the boundary rules
-            const bool ylive = (gk < g.NzY) && !(gk <= kc && gk < nzy);   // fuel value this pass updates
-            if (!live && !ylive) continue;
-            // start the RK operand loads early
-            R ynv[4], accv[4];
-            if (live) {
-    #pragma unroll
-                for (int f = 0; f < 4; f++) {
-                    ynv[f] = a.yn[(size_t)f * N + cg];
-                    accv[f] = rd ? a.acc[(size_t)f * N + cg] : R(0);
-                }
+        }
+    };
+    // a late plane gets a bounded chance to land before the block gives up its shared memory
+    auto settle = [&]() {
+        if (lost >= 0) mbar_wait(sbase + sm.bar + lost * 8, (phases >> lost) & 1, kTmaWaitLimit);
+    };
+    for (int c = ib - 2; c <= ib + 1; c++) fetch(c, c - (ib - 2));
+
+    if (frame && h < CW) {
+        Col q[3];
+#pragma unroll
+        for (int n = 0; n < 3; n++) q[n] = get_col(ib - 2 + n, h - 1);
+#pragma unroll
+        for (int n = 0; n < 3; n++) put_col(ib - 2 + n, h - 1, q[n]);
+    }
+    if (!tma) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    for (int r = 0; r < 4; r++) arrived(r);
+    block_sync();
+    V Y = fuel_at(ib - 1), coef = coef_at(ib - 1);
+
+    // values beyond the walls and second derivatives of T on them, of plane c in the
+    // ring slot at byte offset b: frame threads, a row each
+    const bool has_bot = k0 == 0, has_top = k0 + tk >= Nz;
+    auto walls = [&](int c, uint32_t b) {
+        for (int q = h; q < 2 * CW; q += FR) {
+            const bool lo = q < CW;
+            if (!(lo ? has_bot : has_top)) continue;
+            const int row = lo ? q : q - CW, kw = lo ? 0 : Nz - 1 - k0, st = lo ? (int)E : -(int)E;
+            const uint32_t o = b + SM::s(row - 1, kw), w = sm.wall + (lo ? 0 : 7 * E);
+            auto W = [&](int n) { return sh<const R>(w + n * E); };
+#pragma unroll
+            for (int f = 0; f < 4; f++) {
+                const uint32_t of = o + f * SM::FX;
+                const R f0 = sh<const R>(of);   // the weights' sum is one
+                sh<R>(of - st) = f0 + (W(1) * (sh<const R>(of + st) - f0) + W(2) * (sh<const R>(of + 2 * st) - f0));
             }
-            const size_t oY = 4 * (size_t)N + (size_t)col * g.NzY + gk;
-            R ynY = R(0), accY = R(0);
-            if (ylive) {
-                ynY = a.yn[oY];
-                accY = rd ? a.acc[oY] : R(0);
+            const uint32_t oT = o + 3 * SM::FX, d = sm.corr + (((c & 1) * 2 + (lo ? 0 : 1)) * CW + row) * (VW * E);
+            const int e = VW == 2 && !lo ? (Nz - 1) & 1 : 0;   // the wall cell's place among its thread's cells
+            if (VW == 2) sh<R>(d + (1 - e) * E) = R(0);
+            const R T0 = sh<const R>(oT);   // the weights' sum is zero
+            sh<R>(d + e * E) = W(4) * (sh<const R>(oT + st) - T0) + W(5) * (sh<const R>(oT + 2 * st) - T0) + W(6) * (sh<const R>(oT + 3 * st) - T0);
+        }
+    };
+    if (frame) walls(ib - 1, sm.planeS);
+    block_sync();
+
+    // byte offsets of this thread's cells in the ring slots of planes c-2 .. c+2 and
+    // of the SGS planes c, c-1, c-2, moved on by one slot per iteration
+    const uint32_t endS = SM::RS * sm.planeS + so, endG = SM::RG * sm.planeG + go;
+    uint32_t am2 = endS - sm.planeS, am1 = so, a0 = so + sm.planeS, ap1 = a0 + sm.planeS, ap2 = ap1 + sm.planeS;
+    uint32_t g0 = go, g1 = endG - sm.planeG, g2 = g1 - sm.planeG;
+    int rn = 4;   // ring slot of plane c + 3
+    auto next_plane = [&](int c) {
+        // the plane fetched in this iteration (c + 3) is used from the next one on
+        if (!tma) asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (c + 3 <= ie + 1) arrived(rn);
+        rn = rn == SM::RS - 1 ? 0 : rn + 1;
+        am2 = am1;
+        am1 = a0;
+        a0 = ap1;
+        ap1 = ap2;
+        ap2 += sm.planeS;
+        if (ap2 == endS) ap2 = so;
+        const uint32_t t = g2;
+        g2 = g1;
+        g1 = g0;
+        g0 = t;
+        block_sync();
+    };
+
+    if (frame) {
+#pragma unroll 1
+        for (int c = ib - 1; c <= ie; c++) {
+            if (c + 3 <= ie + 1) fetch(c + 3, rn);
+            if (c + 1 < ie) prefetch_rk(c + 1);
+            V Yn = c_(R(0)), coefn = c_(R(1));
+            Col col = {};
+            if (c < ie) {
+                Yn = fuel_at(c + 1);
+                coefn = coef_at(c + 1);
+                if (h < CW) col = get_col(c + 2, h - 1);
+                if (has_bot || has_top) walls(c + 1, ap1 - so);
             }
-            R kY = R(0);
-            // fuel fraction of the stage input (used only below the column's fuel top)
-            const R Yx = (gk < nzy) ? X[4 * (size_t)N + (size_t)col * g.NzY + gk] : R(0);
-            if (live) {
-                const R *kmw = &t.kr[(kk + 1) * KROW + RKM], *kpw = &t.kr[(kk + 1) * KROW + RKP];
-                const R d2m = t.K(kk, RD2), d20 = t.K(kk, RD2 + 1), d2p = t.K(kk, RD2 + 2);
-                R u, v, w, T;
-                R advU, advV, advW, advT, lapU, lapV, lapW, lapT, Tx, Ty, Tz;
-                if constexpr (TL::PAIRED) {
-                    const float2 UV = t.P(0, ii, jj, kk), WT = t.P(1, ii, jj, kk);
-                    u = UV.x; v = UV.y; w = WT.x; T = WT.y;
-                    // The upwind advection of a field is a weighted sum of its 13
-                    // stencil values and the Laplacian one of 7: with a = max(u,0)/(2dx)
-                    // and b = min(u,0)/(2dx), u+ (3f - 4f_{i-1} + f_{i-2})/(2dx) +
-                    // u- (-3f + 4f_{i+1} - f_{i+2})/(2dx) has weights 3(a-b), -4a, a, 4b, -b;
-                    // in z the two 5-point rows combine as w+ kmw + w- kpw.
-                    const R ax = rmax(u, R(0)) * p.inv2dx, bx = rmin(u, R(0)) * p.inv2dx;
-                    const R ay = rmax(v, R(0)) * p.inv2dy, by = rmin(v, R(0)) * p.inv2dy;
-                    const R wp = rmax(w, R(0)), wm = rmin(w, R(0));
-                    const float2 Cxm = bcast(R(-4) * ax), Cxm2 = bcast(ax), Cxp = bcast(R(4) * bx), Cxp2 = bcast(-bx);
-                    const float2 Cym = bcast(R(-4) * ay), Cym2 = bcast(ay), Cyp = bcast(R(4) * by), Cyp2 = bcast(-by);
-                    const float2 Cz0 = bcast(wp * kmw[0] + wm * kpw[0]), Cz1 = bcast(wp * kmw[1] + wm * kpw[1]);
-                    const float2 Cz3 = bcast(wp * kmw[3] + wm * kpw[3]), Cz4 = bcast(wp * kmw[4] + wm * kpw[4]);
-                    const float2 C0 = bcast(R(3) * (ax - bx) + R(3) * (ay - by) + (wp * kmw[2] + wm * kpw[2]));
-                    const float2 Lx = bcast(p.invdx2), Ly = bcast(p.invdy2), Lzm = bcast(d2m), Lzp = bcast(d2p);
-                    const float2 L0 = bcast(d20 - R(2) * p.invdx2 - R(2) * p.invdy2);
-                    const float2 i2x = bcast(p.inv2dx), i2y = bcast(p.inv2dy), i2z = bcast(t.K(kk, RD1));
-                    auto adv_lap2 = [&](int pr, float2 f0, float2 &adv, float2 &lap, float2 &gx, float2 &gy, float2 &gz) {
-                        const float2 xm = t.P(pr, ii - 1, jj, kk), xp = t.P(pr, ii + 1, jj, kk);
-                        const float2 xm2 = t.P(pr, ii - 2, jj, kk), xp2 = t.P(pr, ii + 2, jj, kk);
-                        const float2 ym = t.P(pr, ii, jj - 1, kk), yp = t.P(pr, ii, jj + 1, kk);
-                        const float2 ym2 = t.P(pr, ii, jj - 2, kk), yp2 = t.P(pr, ii, jj + 2, kk);
-                        const float2 zm2 = t.P(pr, ii, jj, kk - 2), zm = t.P(pr, ii, jj, kk - 1);
-                        const float2 zp = t.P(pr, ii, jj, kk + 1), zp2 = t.P(pr, ii, jj, kk + 2);
-                        float2 s0 = mul2(C0, f0);
-                        s0 = fma2(Cxm, xm, s0);
-                        s0 = fma2(Cxm2, xm2, s0);
-                        s0 = fma2(Cxp, xp, s0);
-                        s0 = fma2(Cxp2, xp2, s0);
-                        s0 = fma2(Cym, ym, s0);
-                        s0 = fma2(Cym2, ym2, s0);
-                        s0 = fma2(Cyp, yp, s0);
-                        s0 = fma2(Cyp2, yp2, s0);
-                        s0 = fma2(Cz0, zm2, s0);
-                        s0 = fma2(Cz1, zm, s0);
-                        s0 = fma2(Cz3, zp, s0);
-                        adv = fma2(Cz4, zp2, s0);
-                        float2 l0 = mul2(L0, f0);
-                        l0 = fma2(Lx, add2(xp, xm), l0);
-                        l0 = fma2(Ly, add2(yp, ym), l0);
-                        l0 = fma2(Lzm, zm, l0);
-                        lap = fma2(Lzp, zp, l0);
-                        gx = mul2(sub2(xp, xm), i2x);
-                        gy = mul2(sub2(yp, ym), i2y);
-                        gz = mul2(sub2(zp, zm), i2z);
-                    };
-                    float2 aUV, lUV, aWT, lWT, gx, gy, gz;
-                    adv_lap2(0, UV, aUV, lUV, gx, gy, gz);
-                    adv_lap2(1, WT, aWT, lWT, gx, gy, gz);
-                    advU = aUV.x; advV = aUV.y; advW = aWT.x; advT = aWT.y;
-                    lapU = lUV.x; lapV = lUV.y; lapW = lWT.x; lapT = lWT.y;
-                    Tx = gx.y; Ty = gy.y; Tz = gz.y;
-                } else {
-                    u = t.S(0, ii, jj, kk); v = t.S(1, ii, jj, kk); w = t.S(2, ii, jj, kk); T = t.S(3, ii, jj, kk);
-                    const R u_plu = rmax(u, R(0)), u_min = rmin(u, R(0));
-                    const R v_plu = rmax(v, R(0)), v_min = rmin(v, R(0));
-                    const R w_plu = rmax(w, R(0)), w_min = rmin(w, R(0));
-                    // advection (upwind) and Laplacian of one field from the shared tile
-                    auto adv_lap = [&](int f, R f0, R &adv, R &lap, R &fx, R &fy, R &fz) {
-                        const R xm = t.S(f, ii - 1, jj, kk), xp = t.S(f, ii + 1, jj, kk);
-                        const R xm2 = t.S(f, ii - 2, jj, kk), xp2 = t.S(f, ii + 2, jj, kk);
-                        const R ym = t.S(f, ii, jj - 1, kk), yp = t.S(f, ii, jj + 1, kk);
-                        const R ym2 = t.S(f, ii, jj - 2, kk), yp2 = t.S(f, ii, jj + 2, kk);
-                        const R zm2 = t.S(f, ii, jj, kk - 2), zm = t.S(f, ii, jj, kk - 1);
-                        const R zp = t.S(f, ii, jj, kk + 1), zp2 = t.S(f, ii, jj, kk + 2);
-                        const R im = (R(3) * f0 - R(4) * xm + xm2) * p.inv2dx;
-                        const R ip = (R(-3) * f0 + R(4) * xp - xp2) * p.inv2dx;
-                        const R jm = (R(3) * f0 - R(4) * ym + ym2) * p.inv2dy;
-                        const R jp = (R(-3) * f0 + R(4) * yp - yp2) * p.inv2dy;
-                        const R km = dz5(kmw, zm2, zm, f0, zp, zp2), kpv = dz5(kpw, zm2, zm, f0, zp, zp2);
-                        adv = (u_plu * im + u_min * ip) + (v_plu * jm + v_min * jp) + (w_plu * km + w_min * kpv);
-                        const R fxx = (xp - R(2) * f0 + xm) * p.invdx2;
-                        const R fyy = (yp - R(2) * f0 + ym) * p.invdy2;
-                        const R fzz = d2m * zm + d20 * f0 + d2p * zp;
-                        lap = fxx + fyy + fzz;
-                        fx = (xp - xm) * p.inv2dx;
-                        fy = (yp - ym) * p.inv2dy;
-                        fz = (zp - zm) * t.K(kk, RD1);
-                    };
-                    R fx, fy, fz;
-                    adv_lap(3, T, advT, lapT, Tx, Ty, Tz);
-                    adv_lap(0, u, advU, lapU, fx, fy, fz);
-                    adv_lap(1, v, advV, lapV, fx, fy, fz);
-                    adv_lap(2, w, advW, lapW, fx, fy, fz);
-                }
-                const R rho = fdiv(p.Trho, T);
-                const Thermo<R> th = thermo(p, smu, sk, T, t.S(3, ii, jj, kk + 1), Yx, gk, nzy, Tx,
-                                            Ty, Tz, lapT, t.K(kk, RDZ), rho);
-                kY = -p.Y_f * th.K_T * th.Y;
-                R kval[4];
-                kval[3] = (a.ph.temperature_convection == 0) ? th.T_RHS_tmp - (u * Tx + v * Ty + w * Tz)
-                                                             : th.T_RHS_tmp - advT;
-                const R mod_U = rsqrt_(u * u + v * v + w * w);
-                kval[0] = th.nu * lapU - advU + (-p.cd * th.Y * mod_U * u);
-                kval[1] = th.nu * lapV - advV + (-p.cd * th.Y * mod_U * v);
-                kval[2] = th.nu * lapW - advW + (fdiv(p.g * (rho - p.rho_inf), rho) - p.cd * th.Y * mod_U * w);
-                // ---- SGS divergence with Van Driest damping (turbulence.cu:255-454)
-                {
-                    const R nu = fdiv(p.mu, rho);
-                    const R inv_avd_nu = fdiv(p.inv_avd, nu);
-                    const R zk = t.K(kk, RZ);
-                    auto zibm = [&](int q, R zz) -> R {
-                        const R d = zz - (R)t.ctopo[q];
-                        return d > R(0) ? d : R(0);
-                    };
-                    const int qxp = TL::cq(ii + 1, jj), qxm = TL::cq(ii - 1, jj);
-                    const int qyp = TL::cq(ii, jj + 1), qym = TL::cq(ii, jj - 1);
-                    R mu_c = t.G(0, ii, jj, kk);
-                    R mu_xp = t.G(0, ii + 1, jj, kk), mu_xm = t.G(0, ii - 1, jj, kk);
-                    R mu_yp = t.G(0, ii, jj + 1, kk), mu_ym = t.G(0, ii, jj - 1, kk);
-                    R mu_kp = t.G(0, ii, jj, kk + 1), mu_km = t.G(0, ii, jj, kk - 1);
-                    // Van Driest factors; where the bound shows them all to be
-                    // exactly 1 the products would not change mu
-                    if (s_vd_bound > VanDriestCut<R>::v * R(1.001) * nu) {
-                        if (*s_vd_zero) {
-                            // columns without friction: the factor of -z_ibm * 0 * inv_avd_nu,
-                            // 1 - exp(-0) = 0 (NaN when 1/nu is not finite, as there)
-                            const R f0 = R(0) * inv_avd_nu, f00 = f0 * f0;
-                            if (t.cut_[cc] == R(0)) {
-                                mu_c *= f00;
-                                mu_kp *= f00;
-                                mu_km *= f00;
-                            }
-                            if (t.cut_[qxp] == R(0)) mu_xp *= f00;
-                            if (t.cut_[qxm] == R(0)) mu_xm *= f00;
-                            if (t.cut_[qyp] == R(0)) mu_yp *= f00;
-                            if (t.cut_[qym] == R(0)) mu_ym *= f00;
-                        }
+            if (c >= ib && h < tj) {
+                // Van Driest bound of the columns around (c, h): see part B
+                const uint32_t oc = col_slot(c) + h + 1, o5[5] = {oc, col_slot(c + 1) + h + 1, col_slot(c - 1) + h + 1, oc + 1, oc - 1};
+                R hmax = R(-1e30), umin = R(1e30);
+                int zero = 0;
+#pragma unroll
+                for (int q = 0; q < 5; q++) {
+                    const R ut = sh<R>(sm.cut_ + o5[q] * E);
+                    if (ut == R(0)) {
+                        zero |= 1 << q;
                     } else {
-                        const R ut0 = t.cut_[cc];
-                        R fc = -zibm(cc, zk) * ut0 * inv_avd_nu;
-                        R fxp_ = -zibm(qxp, zk) * t.cut_[qxp] * inv_avd_nu;
-                        R fxm_ = -zibm(qxm, zk) * t.cut_[qxm] * inv_avd_nu;
-                        R fyp_ = -zibm(qyp, zk) * t.cut_[qyp] * inv_avd_nu;
-                        R fym_ = -zibm(qym, zk) * t.cut_[qym] * inv_avd_nu;
-                        R fkm = -zibm(cc, t.K(kk - 1, RZ)) * ut0 * inv_avd_nu;
-                        R fkp = -zibm(cc, t.K(kk + 1, RZ)) * ut0 * inv_avd_nu;
-                        // A factor is exactly 1 below the cut-off and exactly 0
-                        // where -z+/A is 0 (no height above the terrain, or a
-                        // column without wall friction, as over the hills): only
-                        // a cell with another argument evaluates the exponentials.
-                        if (van_driest_needs_exp(fc) || van_driest_needs_exp(fxp_) || van_driest_needs_exp(fxm_) ||
-                            van_driest_needs_exp(fyp_) || van_driest_needs_exp(fym_) || van_driest_needs_exp(fkm) ||
-                            van_driest_needs_exp(fkp)) {
-                            fc = van_driest(fc);
-                            fxp_ = van_driest(fxp_);
-                            fxm_ = van_driest(fxm_);
-                            fyp_ = van_driest(fyp_);
-                            fym_ = van_driest(fym_);
-                            fkm = van_driest(fkm);
-                            fkp = van_driest(fkp);
-                        } else {
-                            fc = van_driest_exact(fc);
-                            fxp_ = van_driest_exact(fxp_);
-                            fxm_ = van_driest_exact(fxm_);
-                            fyp_ = van_driest_exact(fyp_);
-                            fym_ = van_driest_exact(fym_);
-                            fkm = van_driest_exact(fkm);
-                            fkp = van_driest_exact(fkp);
-                        }
-                        mu_c *= fc * fc;
-                        mu_xp *= fxp_ * fxp_;
-                        mu_xm *= fxm_ * fxm_;
-                        mu_yp *= fyp_ * fyp_;
-                        mu_ym *= fym_ * fym_;
-                        mu_kp *= fkp * fkp;
-                        mu_km *= fkm * fkm;
+                        hmax = rmax(hmax, sh<R>(sm.ctopo + o5[q] * E));
+                        umin = rmin(umin, ut);
                     }
-                    const R S11 = t.G(1, ii, jj, kk), S12 = t.G(2, ii, jj, kk), S13 = t.G(3, ii, jj, kk);
-                    const R S22 = t.G(4, ii, jj, kk), S23 = t.G(5, ii, jj, kk), S33 = t.G(6, ii, jj, kk);
-                    const R wc = t.K(kk, RD1);
-                    const R mu_x = (mu_xp - mu_xm) * p.inv2dx, mu_y = (mu_yp - mu_ym) * p.inv2dy, mu_z = (mu_kp - mu_km) * wc;
-                    const R S11_x = (t.G(1, ii + 1, jj, kk) - t.G(1, ii - 1, jj, kk)) * p.inv2dx;
-                    const R S12_x = (t.G(2, ii + 1, jj, kk) - t.G(2, ii - 1, jj, kk)) * p.inv2dx;
-                    const R S13_x = (t.G(3, ii + 1, jj, kk) - t.G(3, ii - 1, jj, kk)) * p.inv2dx;
-                    const R S21_y = (t.G(2, ii, jj + 1, kk) - t.G(2, ii, jj - 1, kk)) * p.inv2dy;
-                    const R S22_y = (t.G(4, ii, jj + 1, kk) - t.G(4, ii, jj - 1, kk)) * p.inv2dy;
-                    const R S23_y = (t.G(5, ii, jj + 1, kk) - t.G(5, ii, jj - 1, kk)) * p.inv2dy;
-                    const R S31_z = (t.G(3, ii, jj, kk + 1) - t.G(3, ii, jj, kk - 1)) * wc;
-                    const R S32_z = (t.G(5, ii, jj, kk + 1) - t.G(5, ii, jj, kk - 1)) * wc;
-                    const R S33_z = (t.G(6, ii, jj, kk + 1) - t.G(6, ii, jj, kk - 1)) * wc;
-                    const R dU_x = (t.G(7, ii + 1, jj, kk) - t.G(7, ii - 1, jj, kk)) * p.inv2dx;
-                    const R dU_y = (t.G(7, ii, jj + 1, kk) - t.G(7, ii, jj - 1, kk)) * p.inv2dy;
-                    const R dU_z = (t.G(7, ii, jj, kk + 1) - t.G(7, ii, jj, kk - 1)) * wc;
-                    const R div_S_x = S11_x + S21_y + S31_z;
-                    const R div_S_y = S12_x + S22_y + S32_z;
-                    const R div_S_z = S13_x + S23_y + S33_z;
-                    const R inv_rho = fdiv(R(1), rho);
-                    const R sgs_x = R(-2) * (mu_x * S11 + mu_y * S12 + mu_z * S13 + mu_c * div_S_x) * inv_rho;
-                    const R sgs_y = R(-2) * (mu_x * S12 + mu_y * S22 + mu_z * S23 + mu_c * div_S_y) * inv_rho;
-                    const R sgs_z = R(-2) * (mu_x * S13 + mu_y * S23 + mu_z * S33 + mu_c * div_S_z) * inv_rho;
-                    const R sgs_q = -fdiv(mu_x * Tx + mu_y * Ty + mu_z * Tz + mu_c * lapT, rho * p.Pr);
-                    kval[0] += -sgs_x + third(dU_x);
-                    kval[1] += -sgs_y + third(dU_y);
-                    kval[2] += -sgs_z + third(dU_z);
-                    kval[3] -= sgs_q;
                 }
-                // values the column boundary pass needs
-                R *bcs = a.bc + (size_t)col * kBcSlots;
-                if (gk == kc + 1) { bcs[0] = kval[3]; bcs[2] = (gk < nzy) ? kY : R(0); }
-                if (gk == kc + 2) { bcs[1] = kval[3]; bcs[3] = (gk < nzy) ? kY : R(0); }
-                if (gk == Nz - 2) { bcs[4] = kval[0]; bcs[5] = kval[1]; bcs[6] = kval[2]; bcs[7] = kval[3]; }
-                if (gk == Nz - 3) { bcs[8] = kval[0]; bcs[9] = kval[1]; bcs[10] = kval[2]; bcs[11] = kval[3]; }
-    #pragma unroll
+                const uint32_t o = (c & 1) * tj + h;
+                sh<R>(sm.bnd + 2 * o * E) = hmax;
+                sh<R>(sm.bnd + (2 * o + 1) * E) = rmax(umin, R(0)) * p.inv_avd;
+                sh<int>(sm.zero + o * 4) = zero;
+            }
+            if (comp) {
+                const uint32_t s = a0, sp = ap1, sm1 = am1;
+                const V hz = sh<V>(zo + ZD1 * SM::FZ);
+                Grad<V> d[4];
+                V lapT;
+#pragma unroll
                 for (int f = 0; f < 4; f++) {
-                    const size_t o = (size_t)f * N + cg;
-                    a.Xout[o] = rk_update(a.method, a.stage, kval[f], ynv[f], accv[f], an);
-                    if (kp) a.acc[o] = accv[f];
+                    const uint32_t o = f * SM::FX;
+                    const V f0 = sh<V>(s + o);
+                    const auto zn = z_nb<R>(s + o, f0);
+                    const V xm = f0 - sh<V>(sm1 + o), xp = sh<V>(sp + o) - f0, ym = f0 - sh<V>(s + o - SM::ROW_S), yp = sh<V>(s + o + SM::ROW_S) - f0;
+                    const V zm = zn.m1 - f0, zp = zn.p1 - f0;
+                    d[f].x = xp + xm;
+                    d[f].y = yp + ym;
+                    d[f].z = zp - zm;
+                    if (f == 3)
+                        lapT = vfma(sh<V>(zo + (ZD2 + 1) * SM::FZ), zp, vfma(sh<V>(zo + ZD2 * SM::FZ), zm, vfma(cv.ly, yp - ym, cv.lx * (xp - xm)))) +
+                               sh<V>(co + (c & 1) * cstep);
                 }
-            } else if (gk < nzy) {
-                // fuel cell whose velocity and temperature the boundary rules set (top plane)
-                const R T = t.S(3, ii, jj, kk);
-                const R K_T = arrhenius(p, T);
-                kY = -p.Y_f * K_T * Yx;
+                const V T = sh<V>(s + 3 * SM::FX), K_T = arrhenius_v(T);
+                const int nzy = LEAN ? 0 : sh<int2>(sm.cidx + (col_slot(c) + jj + 1) * 8).x;
+                V src, nu, g7;
+                const V Tx = d[3].x * cv.hx, Ty = d[3].y * cv.hy, Tz = d[3].z * hz;
+                sources<R, V, LEAN>(a, cv, Tx, Ty, Tz, lapT, T, Y, K_T, gk, nzy, LEAN ? T : sh<V>(zo + ZDZ * SM::FZ), src, nu, g7);
+                V l2 = sh<V>(zo + ZL * SM::FZ);
+                if (a.coef) l2 = l2 * coef;
+                put_sgs<SM, V>(g0, strain<R, V>(cv, d, hz, T, l2, g7));
             }
-            if (ylive) {
-                const R kv = (gk < nzy) ? kY : R(0);
-                a.Xout[oY] = rk_update(a.method, a.stage, kv, ynY, accY, an);
-                if (kp) a.acc[oY] = accY;
+            if (h < CW && c < ie) put_col(c + 2, h - 1, col);
+            Y = Yn;
+            coef = coefn;
+            next_plane(c);
+        }
+    } else {
+        // ---- the tile ----
+        const bool act = in && gj < Ny && gk < Nz;                  // holds cells of the grid
+        const bool low = act && gk <= a.kcmax + 2, top3 = act && gk + VW > Nz - 3;
+        const uint32_t own = act ? ((uint32_t)gj * (uint32_t)Nz + (uint32_t)gk) * E : 0;
+        // carried from part A of plane c-1 to its part B: right-hand side without the
+        // SGS terms, gradient and Laplacian of T
+        V kA[4], gT[4];
+#pragma unroll
+        for (int f = 0; f < 4; f++) kA[f] = gT[f] = c_(R(0));
+
+#pragma unroll 1
+        for (int c = ib - 1; c <= ie; c++) {
+            if (!tma && c + 3 <= ie + 1) fetch(c + 3, rn);
+            V Yn = c_(R(0)), coefn = c_(R(1));
+            if (c < ie) {
+                Yn = fuel_at(c + 1);
+                coefn = coef_at(c + 1);
             }
+            // ---- A. plane c ----
+            const uint32_t s = a0, sp = ap1, sp2 = ap2, sm1 = am1, sm2 = am2;
+            const V hz = sh<V>(zo + ZD1 * SM::FZ);
+            const V u = sh<V>(s), v = sh<V>(s + SM::FX), w = sh<V>(s + 2 * SM::FX), T = sh<V>(s + 3 * SM::FX);
+            // Upwind advection (pde.cu:341-437) on differences from the cell's value, which leaves no
+            // rounding of the value itself: u+ (3f - 4f_{i-1} + f_{i-2})/(2dx) = u+ (4(f - f_{i-1}) -
+            // (f - f_{i-2}))/(2dx), likewise u-; in z the backward form (weights ZB) carries w+ and the
+            // forward form (ZF) w-, except next to the walls, where one form carries both.
+            const bool rhs = c >= ib && c < ie;   // else only the SGS inputs are wanted
+            // adv holds minus the advection.
+            const V ax = vpos(u) * cv.m_hx, bx = vneg(u) * cv.m_hx, ay = vpos(v) * cv.m_hy, by = vneg(v) * cv.m_hy;
+            const V wb = vfma(sh<V>(zo + ZWW * SM::FZ), w, sh<V>(zo + ZWP * SM::FZ) * vpos(w)), wf = w - wb;
+            const V Czm2 = wb * sh<V>(zo + ZB * SM::FZ), Czm = wb * sh<V>(zo + (ZB + 1) * SM::FZ);
+            const V Czp = wf * sh<V>(zo + (ZF + 1) * SM::FZ), Czp2 = wf * sh<V>(zo + (ZF + 2) * SM::FZ);
+            const V Lzm = sh<V>(zo + ZD2 * SM::FZ), Lzp = sh<V>(zo + (ZD2 + 1) * SM::FZ);
+            Grad<V> d[4];
+            V lap[4], adv[4];
+#pragma unroll
+            for (int f = 0; f < 4; f++) {
+                const uint32_t o = f * SM::FX;
+                const V f0 = f == 0 ? u : f == 1 ? v : f == 2 ? w : T;
+                const auto zn = z_nb<R>(s + o, f0);
+                const V xm = f0 - sh<V>(sm1 + o), xp = sh<V>(sp + o) - f0, ym = f0 - sh<V>(s + o - SM::ROW_S), yp = sh<V>(s + o + SM::ROW_S) - f0;
+                const V zm = zn.m1 - f0, zp = zn.p1 - f0;
+                if (rhs) {
+                    V r = ax * vfma(cv.p4, xm, sh<V>(sm2 + o) - f0);
+                    r = vfma(bx, vfma(cv.p4, xp, f0 - sh<V>(sp2 + o)), r);
+                    r = vfma(ay, vfma(cv.p4, ym, sh<V>(s + o - 2 * SM::ROW_S) - f0), r);
+                    r = vfma(by, vfma(cv.p4, yp, f0 - sh<V>(s + o + 2 * SM::ROW_S)), r);
+                    r = vfma(Czm, zm, r);
+                    r = vfma(Czm2, zn.m2 - f0, r);
+                    r = vfma(Czp, zp, r);
+                    adv[f] = vfma(Czp2, zn.p2 - f0, r);
+                }
+                if (rhs || f == 3) lap[f] = vfma(Lzp, zp, vfma(Lzm, zm, vfma(cv.ly, yp - ym, cv.lx * (xp - xm))));
+                d[f].x = xp + xm;
+                d[f].y = yp + ym;
+                d[f].z = zp - zm;
+            }
+            const uint32_t oq = (uint32_t)(c - 1) * plane + own;
+            const bool upd = act && c > ib;
+            // RK operands of plane c-1, early (what is written to the cut node and the top plane is
+            // lost: k_stage_edge has their values)
+            V yv[4], av[4];
+#pragma unroll
+            for (int f = 0; f < 4; f++) {
+                yv[f] = av[f] = c_(R(0));
+                if constexpr (VEC) {
+                    if (upd && !kstore) yv[f] = *reinterpret_cast<const V *>(&at(a.yn, f, oq));
+                    if (upd && rd) av[f] = *reinterpret_cast<const V *>(&at(a.acc, f, oq));
+                } else {
+#pragma unroll
+                    for (int e = 0; e < VW; e++)
+                        if (upd && gk + e < Nz) {
+                            if (!kstore) set_el(yv[f], e, at(a.yn, f, oq + e * E));
+                            if (rd) set_el(av[f], e, at(a.acc, f, oq + e * E));
+                        }
+                }
+            }
+            lap[3] = lap[3] + sh<V>(co + (c & 1) * cstep);
+            const V K_T = arrhenius_v(T);
+            const int nzy = LEAN ? 0 : sh<int2>(sm.cidx + (col_slot(c) + jj + 1) * 8).x;
+            V src, nu, g7;
+            const V Tx = d[3].x * cv.hx, Ty = d[3].y * cv.hy, Tz = d[3].z * hz;
+            sources<R, V, LEAN>(a, cv, Tx, Ty, Tz, lap[3], T, Y, K_T, gk, nzy, LEAN ? T : sh<V>(zo + ZDZ * SM::FZ), src, nu, g7);
+            V l2 = sh<V>(zo + ZL * SM::FZ);
+            if (a.coef) l2 = l2 * coef;
+            const Sgs<V> q0 = strain<R, V>(cv, d, hz, T, l2, g7);
+            if (comp) put_sgs<SM, V>(g0, q0);
+
+            // ---- B. plane c-1 ----
+            if (c > ib) {
+                int kc = -3;
+                if (low) kc = sh<int2>(sm.cidx + (col_slot(c - 1) + jj + 1) * 8).y;
+                const V Tq = sh<V>(sm1 + 3 * SM::FX), nuq = cv.mu_Trho * Tq;
+                auto G1 = [&](int f) { return sh<V>(g1 + f * SM::FG); };
+                auto G2 = [&](int f) { return sh<V>(g2 + f * SM::FG); };
+                auto Gyp = [&](int f) { return sh<V>(g1 + f * SM::FG + SM::ROW_G); };
+                auto Gym = [&](int f) { return sh<V>(g1 + f * SM::FG - SM::ROW_G); };
+                V mu_c = G1(G_MU), mu_xp = q0.mu, mu_xm = G2(G_MU), mu_yp = Gyp(G_MU), mu_ym = Gym(G_MU), mu_kp, mu_km;
+                if constexpr (VW == 2) {
+                    mu_km.v = make_float2(sh<float>(g1 - 4), mu_c.v.x);
+                    mu_kp.v = make_float2(mu_c.v.y, sh<float>(g1 + 8));
+                } else {
+                    mu_km = sh<V>(g1 - 8);
+                    mu_kp = sh<V>(g1 + 8);
+                }
+                // Van Driest damping (turbulence.cu:255-454): the factor of a point is
+                // 1 - exp(-z_ibm u_tau / (A nu)) with its column's distance and friction and this
+                // cell's nu.  Where the least z_ibm u_tau / A of the columns with friction
+                // exceeds the cut-off times nu, their factors are exactly 1; a column without
+                // friction (u_tau = 0, as over the hills) has the factor 1 - exp(-0) = 0.
+                const uint32_t ob = ((c - 1) & 1) * tj + jj;
+                const R hb = sh<R>(sm.bnd + 2 * ob * E), ub = sh<R>(sm.bnd + (2 * ob + 1) * E);
+                const R zlow = rmax(sh<R>(zo + ZZ * SM::FZ - E) - hb, R(0)) * ub, cutoff = VanDriestCut<R>::v * R(1.001);
+                bool far = zlow > cutoff * el(nuq, 0);
+                if (VW == 2) far = far && zlow > cutoff * el(nuq, 1);
+                far = far || !act;
+                const int zero = sh<int>(sm.zero + ob * 4);
+                if (far && zero) {
+                    const V z0 = c_(R(0)), z1 = c_(R(1));
+                    const V fc = (zero & 1) ? z0 : z1;
+                    mu_c = mu_c * fc;
+                    mu_kp = mu_kp * fc;
+                    mu_km = mu_km * fc;
+                    mu_xp = mu_xp * ((zero & 2) ? z0 : z1);
+                    mu_xm = mu_xm * ((zero & 4) ? z0 : z1);
+                    mu_yp = mu_yp * ((zero & 8) ? z0 : z1);
+                    mu_ym = mu_ym * ((zero & 16) ? z0 : z1);
+                }
+                // the others, few lanes of a warp, with the whole warp: four of them at a
+                // time, a lane for one of the seven points of one of them
+                unsigned near = __ballot_sync(0xffffffffu, !far);
+                while (near) {
+                    const int lane = tid & 31, pt = lane % 7;
+                    unsigned m = near;
+                    int src = 0, rank = -1;   // the cell this lane works for, this lane's own place among the four
+#pragma unroll
+                    for (int n = 0; n < 4; n++) {
+                        const int l = __ffs(m) - 1;
+                        if (n == lane / 7 && l >= 0) src = l;
+                        if (n == 0 || l >= 0) rank = l == lane ? n : rank;
+                        m &= m - 1;
+                    }
+                    near = m;
+                    const V q = vdiv(c_(-p.inv_avd), vshfl(nuq, src));
+                    const int jr = __shfl_sync(0xffffffffu, jj, src), kr = __shfl_sync(0xffffffffu, kk, src);
+                    const uint32_t o = (col_slot(pt == 1 ? c : pt == 2 ? c - 2 : c - 1) + jr + (pt == 3 ? 2 : pt == 4 ? 0 : 1)) * E;
+                    const uint32_t oz = sm.zr + ZZ * SM::FZ + SM::z(kr + (pt == 5 ? 1 : pt == 6 ? -1 : 0));
+                    V zh;
+#pragma unroll
+                    for (int e = 0; e < VW; e++) set_el(zh, e, sh<R>(oz + e * E));
+                    const V f = vd_factor2<R, V>(zh, sh<R>(sm.ctopo + o), sh<R>(sm.cut_ + o), q);
+                    const int from = (rank < 0 ? 0 : rank) * 7;
+                    auto damp = [&](V &mu, int n) {
+                        const V x = vshfl(f, from + n);
+                        if (rank >= 0) mu = mu * x;
+                    };
+                    damp(mu_c, 0);
+                    damp(mu_xp, 1);
+                    damp(mu_xm, 2);
+                    damp(mu_yp, 3);
+                    damp(mu_ym, 4);
+                    damp(mu_kp, 5);
+                    damp(mu_km, 6);
+                }
+                const V mu_x = (mu_xp - mu_xm) * cv.hx, mu_y = (mu_yp - mu_ym) * cv.hy, mu_z = (mu_kp - mu_km) * hz;
+                const V S11 = G1(G_S11), S12 = G1(G_S12), S13 = G1(G_S13), S22 = G1(G_S22), S23 = G1(G_S23), S33 = G1(G_S33);
+                auto zd = [&](int f, V own_v) { return z_diff<R>(g1 + f * SM::FG, own_v); };
+                const V two_inv_rho = cv.two_inv_Trho * Tq;
+                V k[4];
+                V dS = vfma(zd(G_S13, S13), hz, vfma(Gyp(G_S12) - Gym(G_S12), cv.hy, (q0.S11 - G2(G_S11)) * cv.hx));
+                V t = vfma(mu_c, dS, vfma(mu_z, S13, vfma(mu_y, S12, mu_x * S11)));
+                k[0] = vfma(two_inv_rho, t, vfma((q0.g7 - G2(G_Q)) * cv.hx, cv.third, kA[0]));
+                dS = vfma(zd(G_S23, S23), hz, vfma(Gyp(G_S22) - Gym(G_S22), cv.hy, (q0.S12 - G2(G_S12)) * cv.hx));
+                t = vfma(mu_c, dS, vfma(mu_z, S23, vfma(mu_y, S22, mu_x * S12)));
+                k[1] = vfma(two_inv_rho, t, vfma((Gyp(G_Q) - Gym(G_Q)) * cv.hy, cv.third, kA[1]));
+                dS = vfma(zd(G_S33, S33), hz, vfma(Gyp(G_S23) - Gym(G_S23), cv.hy, (q0.S13 - G2(G_S13)) * cv.hx));
+                t = vfma(mu_c, dS, vfma(mu_z, S33, vfma(mu_y, S23, mu_x * S13)));
+                k[2] = vfma(two_inv_rho, t, vfma(zd(G_Q, G1(G_Q)) * hz, cv.third, kA[2]));
+                t = vfma(mu_c, gT[3], vfma(mu_z, gT[2], vfma(mu_y, gT[1], mu_x * gT[0])));
+                k[3] = vfma(cv.inv_Trho_Pr * Tq, t, kA[3]);
+                if (low || top3) {
+                    // k-values the boundary rules extrapolate from
+                    R *bg = a.bc + (size_t)((c - 1) * Ny + gj) * kBcSlots;
+#pragma unroll
+                    for (int e = 0; e < VW; e++) {
+                        const int q = gk + e;
+                        if (q == kc + 1 || q == kc + 2) bg[q - kc - 1] = el(k[3], e);
+                        if (q < kc) {   // below the cut node (pde.cu:88-97)
+#pragma unroll
+                            for (int f = 0; f < 4; f++) set_el(k[f], e, p.dead[f]);
+                        }
+                        if (q == Nz - 2 || q == Nz - 3) {
+#pragma unroll
+                            for (int f = 0; f < 4; f++) bg[(q == Nz - 2 ? 2 : 6) + f] = el(k[f], e);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int f = 0; f < 4; f++) {
+                    const V out = vfma(cv.ar, vfma(cv.cA, av[f], k[f]), yv[f]);
+                    const V acc = vfma(cv.cK, k[f], av[f]);
+                    if constexpr (VEC) {
+                        if (act) *reinterpret_cast<V *>(&const_cast<R &>(at(a.Xout, f, oq))) = out;
+                        if (act && kp) *reinterpret_cast<V *>(&const_cast<R &>(at(a.acc, f, oq))) = acc;
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < VW; e++)
+                            if (act && gk + e < Nz) {
+                                const_cast<R &>(at(a.Xout, f, oq + e * E)) = el(out, e);
+                                if (kp) const_cast<R &>(at(a.acc, f, oq + e * E)) = el(acc, e);
+                            }
+                    }
+                }
+            }
+            // right-hand side of plane c without the SGS terms; buoyancy
+            // g (rho - rho_inf) / rho with rho = T_inf rho_inf / T
+            if (!rhs) {
+#pragma unroll
+                for (int f = 0; f < 4; f++) adv[f] = lap[f] = c_(R(0));   // not used
+            }
+            kA[0] = vfma(nu, lap[0], adv[0]);
+            kA[1] = vfma(nu, lap[1], adv[1]);
+            kA[2] = vfma(cv.g_Tinf, cv.T_inf - T, vfma(nu, lap[2], adv[2]));
+            if (a.ph.temperature_convection == 0) adv[3] = c_(R(-1)) * vfma(w, Tz, vfma(v, Ty, u * Tx));
+            kA[3] = src + adv[3];
+            if constexpr (!LEAN) {
+                const V drag = c_(-p.cd) * Y * vsqrt(vfma(w, w, vfma(v, v, u * u)));   // Y is 0 above the fuel
+                kA[0] = vfma(drag, u, kA[0]);
+                kA[1] = vfma(drag, v, kA[1]);
+                kA[2] = vfma(drag, w, kA[2]);
+            }
+            gT[0] = Tx;
+            gT[1] = Ty;
+            gT[2] = Tz;
+            gT[3] = lap[3];
+            Y = Yn;
+            coef = coefn;
+            next_plane(c);
         }
-        __syncthreads();
-        // ---- 4. cut node and top of the tile's columns, where the two cells
-        //        they extrapolate from are in this tile (their k-values were
-        //        stored to a.bc above); the other columns go to k_stage_bc.
-        for (int q = threadIdx.x; q < TI * TJ; q += NT) {
-            const int ii = q / TJ, jj = q % TJ;
-            const int gi = i0 + ii, gj = j0 + jj;
-            if (gi >= Nx || gj >= Ny) continue;
-            const int col = gi * Ny + gj;
-            const int kc = t.ccut[TL::cq(ii, jj)], nzy = t.cnzy[TL::cq(ii, jj)];
-            if (kc >= k0 && kc < k0 + KZ && bc_cut_in_tile(kc, KZ)) bc_cut_node(a, col, kc, nzy, rd, kp, an);
-            if (Nz - 1 >= k0 && Nz - 1 < k0 + KZ && bc_top_in_tile(Nz, KZ)) bc_top(a, col, rd, kp, an);
+    }
+    settle();
+}
+
+// ---------------------------------------------------------------------------
+// What the fused pass leaves of a stage (pde.cu:14-99, 713-720), eight threads per
+// column: the top plane (threads 0-3, a field each), the cut node (4-7) and the
+// fuel (all).  The k-values they extrapolate from, and their accumulators, are in
+// a.bc.  These cells are few, each a chain of dependent loads: as a kernel of their
+// own all chains run at once, where at the end of each block of the fused pass they
+// cost 75 of its 436 us (256 x 256 x 128 with hills, FP32).  Fuel entries above a
+// column's fuel top never change and are not read, so only the stage that makes
+// the new state copies them.  The thread of the cut node's T also takes the next
+// stage's wall friction velocity, which saves that stage its k_utau.
+template <class R>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? 12 : 8) k_stage_edge(const StageArgs<R> a, int all_fuel)
+{
+    const Geom &g = a.g;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int col = t >> 3, p = t & 7, f = p & 3;
+    if (col >= g.Nx * g.Ny) return;
+    const size_t N = (size_t)g.N, cb = (size_t)col * g.Nz;
+    const int i = col / g.Ny, wc = wrap_p(i, g.Nx - 1) * g.Ny + wrap_p(col - i * g.Ny, g.Ny - 1);
+    const int kc = __ldg(g.cut + wc), nzy = __ldg(g.nzy + wc), nf = all_fuel ? g.NzY : nzy;
+    const bool rd = stage_reads_acc(a.method, a.stage), kp = stage_keeps_acc(a.method, a.stage);
+    const R an = (R)a.a_next;
+    R *bc = a.bc + (size_t)col * kBcSlots;
+    const R *w = a.krow + (size_t)kc * KROW;
+    // the top plane and the cut node: no slip, T extrapolated (loads before stores, which may alias them)
+    const bool top = p < 4, cutT = p == 7;
+    const size_t o = f * N + cb + (top ? g.Nz - 1 : kc);
+    const R y = a.yn[o];
+    R *bacc = bc + (top ? 11 + f : 10);
+    R kv = R(0), acc = R(0), T0 = R(1), u[3] = {R(0), R(0), R(0)}, v[3] = {R(0), R(0), R(0)};
+    const bool utau = cutT && a.make_utau;
+    if (utau) {
+        // for the wall friction velocity: u and v of the cut node keep y_n, the others the
+        // fused pass has written
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const R *src = q == kc ? a.yn : a.Xout;
+            u[q] = src[cb + q];
+            v[q] = src[N + cb + q];
         }
+        if (kc > 0) T0 = a.Xout[3 * N + cb];
+    }
+    if (top || cutT) {
+        kv = top ? a.pr.top_w1 * bc[2 + f] - a.pr.top_w2 * bc[6 + f] : w[RCUT1] * bc[0] - w[RCUT2] * bc[1];
+        if (rd) acc = *bacc;
+    }
+    const R out = rk_update(a.method, a.stage, kv, y, acc, an);
+    a.Xout[o] = out;
+    if ((top || cutT) && kp) *bacc = acc;
+    if (utau) a.utau[col] = utau_of(a, u, v, kc == 0 ? out : T0);
+    for (int k = p; k < nf; k += 8) {
+        // rate -Y_f K(T) Y below the fuel top
+        const size_t oY = 4 * N + (size_t)col * g.NzY + k;
+        auto rate = [&](int q) {
+            return q < nzy ? -a.pr.Y_f * arrhenius(a.pr, a.X[3 * N + (size_t)wc * g.Nz + q]) * a.X[oY + q - k] : R(0);
+        };
+        const R yY = a.yn[oY];
+        R aY = (rd && k < nzy) ? a.acc[oY] : R(0), r = R(0);
+        if (k < nzy) r = k == kc ? w[RCUT1] * rate(kc + 1) - w[RCUT2] * rate(kc + 2) : k < kc ? a.pr.dead[4] : rate(k);
+        a.Xout[oY] = rk_update(a.method, a.stage, r, yY, aY, an);
+        if (kp && k < nzy) a.acc[oY] = aY;
     }
 }
 
-
-// ---------------------------------------------------------------------------
-// Boundary values the fused pass could not complete (pde.cu:14-99): the cut
-// node of the listed columns whose kc+1 / kc+2 lie in the next z-tile, and the
-// top plane when Nz-3 and Nz-1 lie in different z-tiles.  One thread per
-// listed column; the k-values come from the boundary slots.
-template <class R>
-__global__ void __launch_bounds__(128) k_stage_bc(const StageArgs<R> a, int KZ)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= a.nbcfix) return;
-    const int col = a.bcfix[q];
-    const int kc = __ldg(a.g.cut + col), nzy = __ldg(a.g.nzy + col);
-    const R an = (R)a.a_next;
-    const bool rd = stage_reads_acc(a.method, a.stage), kp = stage_keeps_acc(a.method, a.stage);
-    if (!bc_cut_in_tile(kc, KZ)) bc_cut_node(a, col, kc, nzy, rd, kp, an);
-    if (!bc_top_in_tile(a.g.Nz, KZ)) bc_top(a, col, rd, kp, an);
-}
-
-}  // namespace
-
-// Tile shapes of the fused pass: TI x TJ columns of KZ = 8 planes, NT threads.
-// FP32 compiles three block forms, all at 24 or 32 warps per SM: 8x16 columns
-// with 512 threads (two blocks, 64 registers) or 384 threads (two blocks, 80
-// registers), and 8x8 columns with 256 threads (three blocks, 80 registers;
-// more halo work per cell).  The per-context tuner in solver.cu times them on
-// the context's own grid.  (Measured and dropped: 8x16 with 256 threads at 118
-// registers, 16 warps per SM, 3-4% slower; 4x16 and 4x8 tiles.)  FP64: 8x8
-// columns with 512 threads (one block, 124 registers, 16 warps: 8.20 -> 6.09 ms
-// per launch at 512x512x128) or 256 threads (200 registers, 8 warps).
-template <class R, int TI_, int TJ_, int NT_ = 256> struct StageShape {
-    static constexpr int TI = TI_, TJ = TJ_, KZ = 8, NT = NT_;
-    using TL = Tile<R, TI, TJ, KZ>;
-    static size_t smem() { return TL::bytes(); }
-};
-template <class R> struct StageShapes;
-template <> struct StageShapes<float> {
+// Block forms of the fused pass, by the names wf_set_stage_tile takes (the last
+// number is the threads of a block): interior and frame threads, blocks per
+// multiprocessor.
+template <int NT_, int FR_, int NB_> struct StageForm { static constexpr int NT = NT_, FR = FR_, NB = NB_; };
+template <class R> struct StageForms;
+template <> struct StageForms<float> {
     static constexpr int count = 3;
-    static constexpr int ti[3] = {8, 8, 8}, tj[3] = {16, 16, 8}, nt[3] = {512, 384, 256};
+    static constexpr int ti[3] = {8, 8, 8}, tj[3] = {16, 16, 8}, name[3] = {512, 384, 256};
 };
-template <> struct StageShapes<double> {
+template <> struct StageForms<double> {
     static constexpr int count = 2;
-    static constexpr int ti[2] = {8, 8}, tj[2] = {8, 8}, nt[2] = {512, 256};
+    static constexpr int ti[2] = {8, 8}, tj[2] = {8, 8}, name[2] = {512, 256};
 };
-
-// the shape with index idx, as a type, for f(Shape)
-template <class R, class F> cudaError_t with_shape(int idx, F f)
+// f(form) for the form with index idx
+template <class R, class F> cudaError_t with_form(int idx, F f)
 {
     if constexpr (sizeof(R) == 4) {
         switch (idx) {
-        case 0: return f(StageShape<R, 8, 16, 512>());
-        case 1: return f(StageShape<R, 8, 16, 384>());
-        case 2: return f(StageShape<R, 8, 8>());
+        case 0: return f(StageForm<416, 96, 1>());
+        case 1: return f(StageForm<288, 96, 1>());
+        case 2: return f(StageForm<192, 64, 2>());
         default: return cudaErrorInvalidValue;
         }
     } else {
         switch (idx) {
-        case 0: return f(StageShape<R, 8, 8, 512>());
-        case 1: return f(StageShape<R, 8, 8>());
+        case 0: return f(StageForm<416, 96, 1>());
+        case 1: return f(StageForm<160, 96, 2>());
         default: return cudaErrorInvalidValue;
         }
     }
 }
+
+}  // namespace
+
+// Planes of a z-tile: nearly equal tiles of at most 32 planes, multiples of 16
+// bytes, the last with at least 4, so that the top plane and the two below it
+// share a tile, and a wall plane and the three next to it a tile or its halo.
+int stage_tile_k(int Nz)
+{
+    for (int n = (Nz + 31) / 32;; n++) {
+        const int tk = ((Nz + n - 1) / n + 3) / 4 * 4;
+        if ((Nz - 1) % tk >= 3) return tk;
+    }
+}
+
+namespace {
+
+// Shared memory of a block with tj rows.
+template <class R> size_t stage_bytes(int tk, int tj) { return tk > kTileK2 ? StageSmem<R, kTileK>(tj).end : StageSmem<R, kTileK2>(tj).end; }
+
+// Tiling of a grid for blocks of form F on sms multiprocessors: rows per tile and
+// x-planes per block of least cost.  A block takes L + 3 iterations (the two
+// planes around its own, and the first loads); blocks differ (those next to the
+// terrain or the top do more), so several passes of short blocks balance better
+// than one of long ones.  An iteration of a partly filled tile is shorter, but by
+// less than its share of the threads.
+template <class R, class F> StageGrid plan_form(int Nx, int Ny, int Nz, int sms)
+{
+    constexpr int VW = Vec<R>::W;
+    StageGrid s;
+    s.tma = false;
+    s.tk = stage_tile_k(Nz);
+    s.ntk = (Nz + s.tk - 1) / s.tk;
+    int jmax = F::NT / (s.tk / VW);
+    if (jmax > F::FR / 2 - s.tk / VW) jmax = F::FR / 2 - s.tk / VW;
+    while (jmax > 1 && stage_bytes<R>(s.tk, jmax) > (size_t)(227 / F::NB - (F::NB > 1 ? 1 : 0)) * 1024) jmax--;
+    double best = 0.0;
+    s.L = 0;
+    for (int n = (Ny + jmax - 1) / jmax; n <= Ny; n++) {
+        const int tj = (Ny + n - 1) / n;
+        if ((Ny + tj - 1) / tj != n) continue;
+        const double iter = 0.4 + 0.6 * (double)(tj * (s.tk / VW)) / F::NT;
+        for (int m = 1; m <= Nx; m++) {
+            const int L = (Nx + m - 1) / m;
+            if ((Nx + L - 1) / L != m) continue;
+            const long long blocks = (long long)s.ntk * n * m, slots = (long long)F::NB * sms;
+            const double waves = (double)((blocks + slots - 1) / slots);
+            const double cost = (waves + 0.25) * (L + 3) * iter;
+            if (s.L == 0 || cost < best) {
+                best = cost;
+                s.L = L;
+                s.tj = tj;
+                s.ntj = n;
+                s.nti = m;
+            }
+        }
+        if (tj <= 4) break;
+    }
+    return s;
+}
+
+}  // namespace
 
 int g_stage_sms = 0;   // multiprocessors of the device, read at set-up
 
@@ -857,16 +1119,55 @@ template <class R> cudaError_t stage_set_attributes()
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (!e) e = cudaDeviceGetAttribute(&g_stage_sms, cudaDevAttrMultiProcessorCount, dev);
-    for (int q = 0; !e && q < StageShapes<R>::count; q++)
-        e = with_shape<R>(q, [](auto sh) {
-            using SH = decltype(sh);
-            return cudaFuncSetAttribute(k_stage_fused<R, SH::TI, SH::TJ, SH::KZ, SH::NT>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::smem());
+    for (int q = 0; !e && q < StageForms<R>::count; q++)
+        e = with_form<R>(q, [](auto f) {
+            using F = decltype(f);
+            const int most = 227 * 1024;
+            const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+            cudaError_t e = cudaSuccess;
+            auto set = [&](auto kw) {
+                constexpr int KW = decltype(kw)::value;
+                if (!e) e = cudaFuncSetAttribute(k_stage_march<R, F::NT, F::FR, F::NB, KW, true, true>, attr, most);
+                if (!e) e = cudaFuncSetAttribute(k_stage_march<R, F::NT, F::FR, F::NB, KW, false, true>, attr, most);
+                if constexpr (Vec<R>::W > 1) {
+                    if (!e) e = cudaFuncSetAttribute(k_stage_march<R, F::NT, F::FR, F::NB, KW, true, false>, attr, most);
+                    if (!e) e = cudaFuncSetAttribute(k_stage_march<R, F::NT, F::FR, F::NB, KW, false, false>, attr, most);
+                }
+            };
+            set(std::integral_constant<int, kTileK>());
+            set(std::integral_constant<int, kTileK2>());
+            return e;
         });
     return e;
 }
 template cudaError_t stage_set_attributes<double>();
 template cudaError_t stage_set_attributes<float>();
+
+static F2 host_splat(float x)
+{
+    F2 v;
+    v.v = make_float2(x, x);
+    return v;
+}
+static double host_splat(double x) { return x; }
+template <class R> static StageVec<R> stage_vec(const StageArgs<R> &a)
+{
+    const PhysR<R> &p = a.pr;
+    const bool kstore = a.method == 3, last = stage_reads_acc(a.method, a.stage) && !stage_keeps_acc(a.method, a.stage);
+    auto s = [](R x) { return host_splat(x); };
+    StageVec<R> q;
+    q.hx = s(p.inv2dx); q.hy = s(p.inv2dy); q.lx = s(p.invdx2); q.ly = s(p.invdy2);
+    q.c12 = s(p.c12); q.c4 = s(p.c4); q.kT = s(p.kT); q.inv_Trho_cp = s(p.inv_Trho_cp); q.H_C_cp = s(p.H_C_cp);
+    q.mu_Trho = s(p.mu_Trho); q.Trho = s(p.Trho); q.two_inv_Trho = s(p.two_inv_Trho); q.inv_Trho_Pr = s(p.inv_Trho_Pr);
+    q.g_Tinf = s(p.g_Tinf); q.T_inf = s(p.T_inf);
+    q.third = s(R(1.0 / 3.0)); q.m_third = s(R(-1.0 / 3.0)); q.half = s(R(0.5)); q.p4 = s(R(4));
+    q.m_hx = s(-p.inv2dx); q.m_hy = s(-p.inv2dy);
+    // RK update out = ar (k + cA acc) + y_n, acc' = acc + cK k (rk_update)
+    q.ar = s(kstore ? R(1) : (R)a.a_next);
+    q.cA = s(last ? R(1) : R(0));
+    q.cK = s(a.method == 2 && a.stage > 1 && a.stage < 4 ? R(2) : R(1));
+    return q;
+}
 
 template <class R> cudaError_t launch_stage(const StageArgs<R> &a, cudaStream_t s, cudaEvent_t *ev)
 {
@@ -876,82 +1177,87 @@ template <class R> cudaError_t launch_stage(const StageArgs<R> &a, cudaStream_t 
                                                   a.closure_wait);
         if (e) return e;
     }
-    k_utau<R><<<(ncol + 127) / 128, 128, 0, s>>>(a);
+    if (!a.have_utau) k_utau<R><<<(ncol + 127) / 128, 128, 0, s>>>(a);
     if (ev) cudaEventRecord(ev[0], s);
-    cudaError_t e = with_shape<R>(a.tile, [&](auto sh) {
-        using SH = decltype(sh);
-        const int ntk = (a.g.Nz + SH::KZ - 1) / SH::KZ, ntj = (a.g.Ny + SH::TJ - 1) / SH::TJ;
-        const int nti = (a.g.Nx + SH::TI - 1) / SH::TI;
-        const int w = SH::TJ == 16 ? 0 : 1;
-        CUtensorMap m, myn, macc;
-        const void *src = (sizeof(R) == 4) ? a.tmap[w] : nullptr;
-        const void *pyn = (sizeof(R) == 4) ? a.pmap_yn[w] : nullptr, *pacc = (sizeof(R) == 4) ? a.pmap_acc[w] : nullptr;
-        if (src) memcpy(&m, src, sizeof(m));
-        else memset(&m, 0, sizeof(m));
-        const bool pf = pyn && pacc;
-        if (pf) {
-            memcpy(&myn, pyn, sizeof(myn));
-            memcpy(&macc, pacc, sizeof(macc));
-        } else {
-            memset(&myn, 0, sizeof(myn));
-            memset(&macc, 0, sizeof(macc));
-        }
-        k_stage_fused<R, SH::TI, SH::TJ, SH::KZ, SH::NT><<<ntk * ntj * nti, SH::NT, SH::smem(), s>>>(
-            a, m, myn, macc, src ? 1 : 0, pf ? 1 : 0, ntk, ntj, nti);
+    const bool lean = a.ph.sutherland_viscosity != 1 && a.ph.sutherland_conductivity != 1 && a.ph.alpha_s * a.ph.sigma_s == 0.0;
+    const StageVec<R> cv = stage_vec(a);
+    cudaError_t e = with_form<R>(a.tile, [&](auto f) {
+        using F = decltype(f);
+        StageGrid sg = a.grid;
+        CUtensorMap m[2];   // X by tiles and by rows
+        memset(m, 0, sizeof(m));
+        sg.tma = a.tmap[0] && a.tmap[1];
+        for (int q = 0; q < 2 && sg.tma; q++) memcpy(&m[q], a.tmap[q], sizeof(m[q]));
+        const int blocks = sg.ntk * sg.ntj * sg.nti, threads = F::NT + F::FR;
+        const size_t smem = stage_bytes<R>(sg.tk, sg.tj);
+        auto go = [&](auto kw, auto lean_, auto vec_) {
+            k_stage_march<R, F::NT, F::FR, F::NB, decltype(kw)::value, decltype(lean_)::value, decltype(vec_)::value>
+                <<<blocks, threads, smem, s>>>(a, cv, sg, m[0], m[1]);
+        };
+        auto go_kw = [&](auto kw) {
+            if (Vec<R>::W == 1 || a.g.Nz % Vec<R>::W == 0) {   // a thread's cells are one aligned access
+                if (lean) go(kw, std::true_type(), std::true_type());
+                else go(kw, std::false_type(), std::true_type());
+            } else if constexpr (Vec<R>::W > 1) {
+                if (lean) go(kw, std::true_type(), std::false_type());
+                else go(kw, std::false_type(), std::false_type());
+            }
+        };
+        if (sg.tk > kTileK2) go_kw(std::integral_constant<int, kTileK>());
+        else go_kw(std::integral_constant<int, kTileK2>());
         return cudaSuccess;
     });
     if (e) return e;
     if (ev) cudaEventRecord(ev[1], s);
-    if (a.nbcfix > 0) k_stage_bc<R><<<(a.nbcfix + 127) / 128, 128, 0, s>>>(a, 8);
+    const bool last = a.method == 3 || !stage_keeps_acc(a.method, a.stage);
+    k_stage_edge<R><<<(unsigned)((8 * (size_t)ncol + 127) / 128), 128, 0, s>>>(a, last);
     if (ev) cudaEventRecord(ev[2], s);
     return cudaGetLastError();
 }
 
-int stage_tile_planes(int precision) { (void)precision; return 8; }
+StageGrid stage_plan(int precision, int form, int Nx, int Ny, int Nz)
+{
+    StageGrid sg;
+    const int sms = g_stage_sms;
+    if (precision == 0) with_form<double>(form, [&](auto f) { sg = plan_form<double, decltype(f)>(Nx, Ny, Nz, sms); return cudaSuccess; });
+    else with_form<float>(form, [&](auto f) { sg = plan_form<float, decltype(f)>(Nx, Ny, Nz, sms); return cudaSuccess; });
+    return sg;
+}
 
-bool stage_tensor_map(void *out, const float *X, int Nx, int Ny, int Nz, int TI, int TJ, void *encode_fn)
+bool stage_tensor_map(void *out, const void *X, int precision, int Nx, int Ny, int Nz, int rows, void *encode_fn)
 {
-    if (!encode_fn || Nz % 4 != 0 || (reinterpret_cast<uintptr_t>(X) & 15) != 0) return false;
+    const size_t E = precision == 0 ? 8 : 4;
+    if (!encode_fn || Nz * E % 16 != 0 || (reinterpret_cast<uintptr_t>(X) & 15) != 0) return false;
     using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    const cuuint64_t dims[4] = {(cuuint64_t)Nz, (cuuint64_t)Ny, (cuuint64_t)Nx, 4};
-    const cuuint64_t strides[3] = {(cuuint64_t)Nz * 4, (cuuint64_t)Ny * Nz * 4, (cuuint64_t)Nx * Ny * Nz * 4};
-    const cuuint32_t box[4] = {16, (cuuint32_t)(TJ + 4), (cuuint32_t)(TI + 4), 4};
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    const cuuint64_t dims[4] = {(cuuint64_t)Nz, 4, (cuuint64_t)Ny, (cuuint64_t)Nx};
+    const cuuint64_t strides[3] = {(cuuint64_t)Nx * Ny * Nz * E, Nz * E, (cuuint64_t)Ny * Nz * E};
+    const bool wide = stage_tile_k(Nz) > kTileK2;
+    const int px = precision == 0 ? (wide ? StageSmem<double, kTileK>::PX : StageSmem<double, kTileK2>::PX)
+                                  : (wide ? StageSmem<float, kTileK>::PX : StageSmem<float, kTileK2>::PX);
+    const cuuint32_t box[4] = {(cuuint32_t)px, 4, (cuuint32_t)rows, 1}, estr[4] = {1, 1, 1, 1};
     const CUresult r = reinterpret_cast<Encode>(encode_fn)(
-        reinterpret_cast<CUtensorMap *>(out), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(X), dims, strides,
-        box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        reinterpret_cast<CUtensorMap *>(out), precision == 0 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
+        const_cast<void *>(X), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
 }
-bool stage_cell_map(void *out, const float *X, int Nx, int Ny, int Nz, int TI, int TJ, void *encode_fn)
-{
-    if (!encode_fn || Nz % 4 != 0 || (reinterpret_cast<uintptr_t>(X) & 15) != 0) return false;
-    using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    const cuuint64_t dims[4] = {(cuuint64_t)Nz, (cuuint64_t)Ny, (cuuint64_t)Nx, 4};
-    const cuuint64_t strides[3] = {(cuuint64_t)Nz * 4, (cuuint64_t)Ny * Nz * 4, (cuuint64_t)Nx * Ny * Nz * 4};
-    const cuuint32_t box[4] = {8, (cuuint32_t)TJ, (cuuint32_t)TI, 4};
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
-    const CUresult r = reinterpret_cast<Encode>(encode_fn)(
-        reinterpret_cast<CUtensorMap *>(out), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(X), dims, strides,
-        box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS;
-}
-int stage_tile_count(int precision) { return precision == 0 ? StageShapes<double>::count : StageShapes<float>::count; }
+
+// Measured at 512 x 512 x 128 FP32 (ms per launch): 1.19 / 1.25 / 1.11; at
+// 256 x 256 x 128 FP64: 0.69 / 0.86.  On small grids the forms are within 10%.
+int stage_default_form(int precision) { return precision == 0 ? 0 : 2; }
+int stage_tile_count(int precision) { return precision == 0 ? StageForms<double>::count : StageForms<float>::count; }
 void stage_tile_shape(int precision, int idx, int *ti, int *tj, int *nt)
 {
     if (precision == 0) {
-        *ti = StageShapes<double>::ti[idx];
-        *tj = StageShapes<double>::tj[idx];
-        if (nt) *nt = StageShapes<double>::nt[idx];
+        *ti = StageForms<double>::ti[idx];
+        *tj = StageForms<double>::tj[idx];
+        if (nt) *nt = StageForms<double>::name[idx];
     } else {
-        *ti = StageShapes<float>::ti[idx];
-        *tj = StageShapes<float>::tj[idx];
-        if (nt) *nt = StageShapes<float>::nt[idx];
+        *ti = StageForms<float>::ti[idx];
+        *tj = StageForms<float>::tj[idx];
+        if (nt) *nt = StageForms<float>::name[idx];
     }
 }
 

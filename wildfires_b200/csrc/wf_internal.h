@@ -69,6 +69,9 @@ template <class R> struct PhysR {
     R T_inf, c_p, rho_inf, cd, g, c12, c4, Pr, inv_avd;
     R T_min, T_max, Y_min, Y_max;
     R mu_Trho, inv_Trho_cp, H_C_cp;     // mu/(T_inf rho_inf), 1/(T_inf rho_inf c_p), H_C/c_p
+    R dead[5];                          // u, v, w, T, Y of dead nodes
+    R top_w1, top_w2;                   // top-plane extrapolation weights (Phys)
+    R g_Tinf, two_inv_Trho, inv_Trho_Pr; // g/T_inf, 2/(T_inf rho_inf), 1/(T_inf rho_inf Pr)
 };
 
 // Per-k row of z-stencil weights in the stencil precision (branch-free
@@ -82,6 +85,7 @@ enum KRow {
     RDEL2 = 15, // Smagorinsky length squared
     RZ = 16,    // z_k
     RDD2 = 17,  // (dx dy dz_k)^(2/3): the filter width squared (learned closure)
+    RCUT1 = 18, RCUT2 = 19, // extrapolation to a cut node k from k+1 and k+2: RCUT1 f_{k+1} - RCUT2 f_{k+2}
     KROW = 20
 };
 
@@ -97,9 +101,18 @@ struct Geom {
     const int *cut;             // [Nx*Ny] cut node per column
 };
 
-// Per-column values the boundary pass needs from the stage pass:
-// T,Y at cut+1, cut+2 (4) and u,v,w,T at Nz-2, Nz-3 (8).
-constexpr int kBcSlots = 12;
+// Per-column values of the boundary rules: k-values of T at cut+1, cut+2 (2) and
+// of u, v, w, T at Nz-2, Nz-3 (8), which they extrapolate from, and the RK
+// accumulators of T at the cut node (1) and of u, v, w, T at the top (4).
+constexpr int kBcSlots = 15;
+
+// Tiling of a grid for the fused stage pass.
+struct StageGrid {
+    int tj, tk;          // rows and planes of a tile
+    int ntj, ntk, nti;   // tiles in j and k, blocks along x
+    int L;               // x-planes of a block
+    bool tma;            // state planes arrive by TMA
+};
 
 template <class R>
 struct StageArgs {
@@ -122,17 +135,14 @@ struct StageArgs {
     const float *theta;    // closure parameters on the device
     int *closure_err;      // set by the closure kernel when a tensor-core wait times out
     int closure_wait;      // polls of each tensor-core completion wait
-    const int *bcfix;      // columns whose cut node or top the fused pass leaves to k_stage_bc
-    int nbcfix;
-    int tile;              // tile shape of the fused pass (index into the compiled shapes)
-    // FP32: host copies of the TMA tensor maps (CUtensorMap) of X for the tile
-    // boxes of 16-column and 8-column tiles, or nullptr (tiles loaded by cp.async)
+    int kcmax;             // highest cut node of the grid
+    bool have_utau;        // utau holds the friction velocity of X already (from the stage that made X)
+    bool make_utau;        // leave that of Xout for the next stage
+    int tile;              // block form of the fused pass (index into the compiled forms)
+    StageGrid grid;        // tiling of the grid for that form
+    // host copies of the TMA tensor maps (CUtensorMap) of X, by tiles and by rows; nullptr: planes copied by cp.async
     const void *tmap[2];
-    // FP32: host copies of the tensor maps of yn and acc for the boxes of the tile's
-    // own cells (16- and 8-column tiles), or nullptr: the stage kernel prefetches
-    // its RK operands into L2 with them while it loads and evaluates its tile
-    const void *pmap_yn[2], *pmap_acc[2];
-    int *kerr;             // set by a stage kernel whose bounded wait for its tile gave up
+    int *kerr;             // set by a stage kernel whose bounded wait for a plane gave up
 };
 
 // Learned closure (closure.cu).
@@ -152,17 +162,15 @@ cudaError_t launch_adam(float *theta, float *m, float *v, const float *g, int st
 // ev (optional): one event recorded after each of the 3 kernels, for profiling.
 template <class R> cudaError_t launch_stage(const StageArgs<R> &a, cudaStream_t s, cudaEvent_t *ev = nullptr);
 template <class R> cudaError_t stage_set_attributes();
-int stage_tile_planes(int precision);   // z planes of a fused-stage tile
-// TMA tensor map (CUtensorMap) of a packed FP32 state for the FP32 tile box of
-// a TI x TJ tile (dims k, j, i, field = Nz, Ny, Nx, 4; box 16 x TJ+4 x TI+4 x 4,
-// 64-byte swizzle); false when the grid cannot be described (column length not a
-// multiple of 4) or the driver call fails.  encode_fn: cuTensorMapEncodeTiled.
-bool stage_tensor_map(void *out, const float *X, int Nx, int Ny, int Nz, int TI, int TJ, void *encode_fn);
-// map of the same buffer for boxes of a tile's own cells (8 planes x TJ x TI x 4 fields)
-bool stage_cell_map(void *out, const float *X, int Nx, int Ny, int Nz, int TI, int TJ, void *encode_fn);
-// Tile shapes compiled for the fused pass (all with the same z planes, so the
-// boundary-column list does not depend on the choice): count and TI x TJ.
+// Tiling for a block form (after stage_set_attributes).
+StageGrid stage_plan(int precision, int form, int Nx, int Ny, int Nz);
+// TMA tensor map (CUtensorMap) of the u, v, w, T of a packed state (dims k, field, j, i; box: `rows` rows of a tile
+// with the halo in k, four fields); false when the columns are no multiple of 16 bytes or the driver call fails.
+// encode_fn: cuTensorMapEncodeTiled.
+bool stage_tensor_map(void *out, const void *X, int precision, int Nx, int Ny, int Nz, int rows, void *encode_fn);
+// Block forms compiled for the fused pass: count and name (TI x TJ, threads) of each.
 int stage_tile_count(int precision);
+int stage_default_form(int precision);
 void stage_tile_shape(int precision, int idx, int *ti, int *tj, int *nt = nullptr);
 
 template <class R>
