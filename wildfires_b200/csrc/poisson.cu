@@ -683,6 +683,112 @@ __global__ void __launch_bounds__(128, 8) k_p_tridiag(double2 *__restrict__ G, c
     }
 }
 
+// P3 where the systems are too few to hide k_p_tridiag's latency: the plain Thomas
+// algorithm with the diagonal u of the forward sweep kept in shared memory and its
+// right-hand sides in G (in L2 at these sizes), so nothing is evaluated twice.
+// The quotients by u are products with 1 / u corrected by their remainder, so
+// they round as divisions do (a plain product loses a digit: for the long waves
+// the elimination is exact where l = a / u is, 1.2e-14 against 1.3e-15 on
+// 257 x 200 x 64), and in the back substitution 1 / u is off the serial chain.  Two
+// threads share a system (real and imaginary part), which doubles the threads and
+// keeps their accesses contiguous; the loads of kThomasAhead planes are in flight
+// while the planes before them are eliminated.  Rows, and what the reference adds
+// to the first and last, as in k_p_tridiag.
+constexpr int kThomasAhead = 8;
+constexpr int kThomasThreads = 64;
+constexpr int kThomasMaxPlanes = 256;   // 256 x 8 bytes x 32 systems = 64 KB, three blocks per SM
+
+// v / u with rec = 1 / u
+__device__ __forceinline__ double quotient(double v, double u, double rec)
+{
+    const double q = v * rec;
+    return fma(fma(-q, u, v), rec, q);
+}
+
+__global__ void __launch_bounds__(kThomasThreads) k_p_thomas(double *__restrict__ G, const double *__restrict__ kx2,
+                                                             const double *__restrict__ ky2, const double *__restrict__ zt,
+                                                             int n0, int h1, int nk)
+{
+    extern __shared__ double2 smem[];
+    constexpr int T = kThomasThreads;
+    const int t = threadIdx.x;
+    double *us = reinterpret_cast<double *>(smem);       // [nk][T/2]
+    double *za = us + (size_t)nk * (T / 2), *zc = za + nk, *zD = zc + nk;   // rows' sub- and superdiagonal, D
+    for (int q = t; q < 3 * nk; q += T) za[q] = zt[q];
+    const int r = blockIdx.x, s = blockIdx.y * (T / 2) + (t >> 1);
+    const bool act = s < h1;
+    const double kk2 = kx2[r] + ky2[act ? s : 0];
+    const double b0 = zt[3 * nk], half_dz0 = zt[3 * nk + 3], cl = zt[3 * nk + 4];
+    const double c0 = zt[3 * nk + 1] - half_dz0 * kk2 - zt[3 * nk + 2];
+    const size_t stride = 2 * (size_t)n0 * h1;
+    double *g = G + 2 * ((size_t)r * h1 + (act ? s : 0)) + (t & 1);
+    // row 0 uses the source of slice 1; the last row subtracts the top pressure
+    // divided by its coupling coefficient
+    double nx[kThomasAhead];
+#pragma unroll
+    for (int q = 0; q < kThomasAhead; q++)
+        if (q < nk) nx[q] = g[stride * (q == 0 ? 1 : q)];
+    const double pt = g[stride * nk];
+    __syncthreads();
+    double u = b0, rec = 1.0 / b0, y = half_dz0 * nx[0];
+    if (act) g[0] = y;
+    if (!(t & 1)) us[t >> 1] = u;
+    for (int q0 = 0; q0 < nk; q0 += kThomasAhead) {
+        double d[kThomasAhead];
+#pragma unroll
+        for (int q = 0; q < kThomasAhead; q++) {
+            d[q] = nx[q];
+            if (q0 + kThomasAhead + q < nk) nx[q] = g[stride * (q0 + kThomasAhead + q)];
+        }
+#pragma unroll
+        for (int q = 0; q < kThomasAhead; q++) {
+            const int k = q0 + q;
+            if (k == 0) continue;
+            if (k >= nk) break;
+            const double l = quotient(za[k - 1], u, rec);
+            u = fma(-l, k == 1 ? c0 : zc[k - 1], -(kk2 + zD[k]));
+            rec = 1.0 / u;
+            if (k == nk - 1) d[q] -= pt / cl;
+            y = fma(-l, y, d[q]);
+            if (act) g[stride * k] = y;
+            if (!(t & 1)) us[k * (T / 2) + (t >> 1)] = u;
+        }
+    }
+    __syncwarp();
+    double x = quotient(y, u, rec);
+    if (act) g[stride * (nk - 1)] = x;
+#pragma unroll
+    for (int q = 0; q < kThomasAhead; q++)
+        if (nk - 2 - q >= 0) nx[q] = g[stride * (nk - 2 - q)];
+    for (int k0 = nk - 2; k0 >= 0; k0 -= kThomasAhead) {
+        double d[kThomasAhead];
+#pragma unroll
+        for (int q = 0; q < kThomasAhead; q++) {
+            d[q] = nx[q];
+            if (k0 - kThomasAhead - q >= 0) nx[q] = g[stride * (k0 - kThomasAhead - q)];
+        }
+#pragma unroll
+        for (int q = 0; q < kThomasAhead; q++) {
+            const int k = k0 - q;
+            if (k < 0) break;
+            const double uk = us[k * (T / 2) + (t >> 1)], rk = 1.0 / uk;
+            x = quotient(fma(-(k == 0 ? c0 : zc[k]), x, d[q]), uk, rk);
+            if (act) g[stride * k] = x;
+        }
+    }
+}
+// One solve (us, k_p_tridiag / k_p_thomas): 33 x 33 x 16 18.7 / 10.2, 64 x 64 x 144 97 / 41,
+// 128 x 128 x 64 60 / 25, 160 x 128 x 48 47 / 21, 257 x 200 x 64 64 / 31, 256 x 256 x 128
+// 130 / 78, 300 x 260 x 64 64 / 39, 512 x 256 x 128 160 / 121, 512 x 512 x 64 102 / 90 and,
+// past the line, 512 x 512 x 128 200 / 205: there the systems alone fill the GPU and the
+// right-hand sides no longer stay in L2.
+constexpr long long kThomasMaxCells = 12000000;   // complex values of G, 192 MB
+bool use_thomas(int n0, int h1, int nk)
+{
+    return nk <= kThomasMaxPlanes && (long long)n0 * h1 * nk <= kThomasMaxCells;
+}
+size_t thomas_smem(int nk) { return (size_t)nk * (kThomasThreads * 4 + 24); }
+
 // P5: inverse FFT in y of packed slice pairs, normalisation, write p and the
 // periodic duplicate planes (pressure.cu:392-416, deterministic here).
 template <class E, class R>
@@ -910,6 +1016,7 @@ template <class R> cudaError_t poisson_set_attributes()
     if (!e) e = cudaDeviceGetAttribute(&g_poisson_sms, cudaDevAttrMultiProcessorCount, dev);
     if (!e) e = set_attributes_for<R, kMinL>();
     if (!e) e = set_pr_attributes_all<R>(PrPlans{});
+    if (!e) e = cudaFuncSetAttribute(k_p_thomas, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)thomas_smem(kThomasMaxPlanes));
     return e;
 }
 template cudaError_t poisson_set_attributes<double>();
@@ -927,7 +1034,11 @@ cudaError_t launch_poisson_impl(const PoissonArgs<R> &a, const double *zt, cudaS
     if ((e = by_engine<LaunchFx<false>, kRadixFft>(a.fx, G, a.fx, ns, n0, h1, s))) return e;
     if (ev) cudaEventRecord(ev[1], s);
     if (nk > kSeg * kMaxSeg) return cudaErrorInvalidValue;
-    k_p_tridiag<<<dim3(n0, (h1 + 127) / 128), 128, 0, s>>>(a.G, a.kx2, a.ky2, zt, n0, h1, nk);
+    if (use_thomas(n0, h1, nk))
+        k_p_thomas<<<dim3(n0, (h1 + kThomasThreads / 2 - 1) / (kThomasThreads / 2)), kThomasThreads, thomas_smem(nk), s>>>(
+            reinterpret_cast<double *>(a.G), a.kx2, a.ky2, zt, n0, h1, nk);
+    else
+        k_p_tridiag<<<dim3(n0, (h1 + 127) / 128), 128, 0, s>>>(a.G, a.kx2, a.ky2, zt, n0, h1, nk);
     if (ev) cudaEventRecord(ev[2], s);
     ns = nk;
     if ((e = by_engine<LaunchFx<true>, kRadixFft>(a.fx, G, a.fx, ns, n0, h1, s))) return e;
