@@ -1257,7 +1257,7 @@ wf_status choose_tile(wf_ctx *c)
     if (c->tile_set) return WF_OK;
     c->tile_set = true;
     const int prec = c->prec == WF_FP64 ? 0 : 1, count = stage_tile_count(prec);
-    c->tile = stage_default_form(prec);
+    c->tile = stage_default_form(prec, c->N);
     if (const char *env = getenv("WF_STAGE_TILE")) {
         int ti = 0, tj = 0, nt = 0;
         const int got = sscanf(env, "%dx%d/%d", &ti, &tj, &nt);   // TIxTJ, optionally /threads

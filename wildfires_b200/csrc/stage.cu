@@ -1074,7 +1074,9 @@ template <class R> size_t stage_bytes(int tk, int tj) { return tk > kTileK2 ? St
 // planes around its own, and the first loads); blocks differ (those next to the
 // terrain or the top do more), so several passes of short blocks balance better
 // than one of long ones.  An iteration of a partly filled tile is shorter, but by
-// less than its share of the threads.
+// less than its share of the threads.  A grid that does not fill the machine is
+// charged for part of what it takes of it: short blocks repeat the planes around
+// them, and the rest is there for other members or contexts.
 template <class R, class F> StageGrid plan_form(int Nx, int Ny, int Nz, int sms)
 {
     constexpr int VW = Vec<R>::W;
@@ -1096,7 +1098,7 @@ template <class R, class F> StageGrid plan_form(int Nx, int Ny, int Nz, int sms)
             if ((Nx + L - 1) / L != m) continue;
             const long long blocks = (long long)s.ntk * n * m, slots = (long long)F::NB * sms;
             const double waves = (double)((blocks + slots - 1) / slots);
-            const double cost = (waves + 0.25) * (L + 3) * iter;
+            const double cost = (blocks < slots ? 0.6 + 0.65 * (double)blocks / slots : waves + 0.25) * (L + 3) * iter;
             if (s.L == 0 || cost < best) {
                 best = cost;
                 s.L = L;
@@ -1244,9 +1246,11 @@ bool stage_tensor_map(void *out, const void *X, int precision, int Nx, int Ny, i
     return r == CUDA_SUCCESS;
 }
 
-// Measured at 512 x 512 x 128 FP32 (ms per launch): 1.19 / 1.25 / 1.11; at
-// 256 x 256 x 128 FP64: 0.69 / 0.86.  On small grids the forms are within 10%.
-int stage_default_form(int precision) { return precision == 0 ? 0 : 2; }
+// Measured at 512 x 512 x 128 FP32 (ms per launch): 1.19 / 1.25 / 1.11; FP64 at
+// 256 x 256 x 128 0.69 / 0.86, at 201 x 150 x 45 0.22 / 0.26, at 33 x 33 x 16 0.021 / 0.019
+// (blocks of 512 threads hold a whole multiprocessor each, however few of their
+// threads a small grid uses).
+int stage_default_form(int precision, long long cells) { return precision == 0 ? (cells < 200000 ? 1 : 0) : 2; }
 int stage_tile_count(int precision) { return precision == 0 ? StageForms<double>::count : StageForms<float>::count; }
 void stage_tile_shape(int precision, int idx, int *ti, int *tj, int *nt)
 {

@@ -170,7 +170,7 @@ StageGrid stage_plan(int precision, int form, int Nx, int Ny, int Nz);
 bool stage_tensor_map(void *out, const void *X, int precision, int Nx, int Ny, int Nz, int rows, void *encode_fn);
 // Block forms compiled for the fused pass: count and name (TI x TJ, threads) of each.
 int stage_tile_count(int precision);
-int stage_default_form(int precision);
+int stage_default_form(int precision, long long cells);
 void stage_tile_shape(int precision, int idx, int *ti, int *tj, int *nt = nullptr);
 
 template <class R>
