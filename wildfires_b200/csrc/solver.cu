@@ -1249,7 +1249,7 @@ wf_status finish_upload(wf_ctx *c)
 }
 
 // Block form of the fused stage pass for this context: WF_STAGE_TILE=TIxTJ[/threads]
-// in the environment forces one, otherwise the one stage_default_form gives.
+// in the environment forces one, otherwise the one stage_default_form gives for the grid.
 // Every form gives bit-identical results: a cell's arithmetic does not depend
 // on the tiling.
 wf_status choose_tile(wf_ctx *c)
@@ -1950,18 +1950,20 @@ __global__ void k_zero_fuel_above(double *R, const int *__restrict__ nzy, int nc
     if (k >= nzy[col]) R[t] = 0.0;
 }
 
-// Packed FP64 device state -> stencil-precision device state, and back, on the
-// context's stream (no host copy).
-wf_status put_state_dev(wf_ctx *c, void *dst, const double *src)
+// Packed FP64 device state (or n of its values) -> stencil-precision device state, and
+// back, on the context's stream (no host copy).
+wf_status put_values_dev(wf_ctx *c, void *dst, const double *src, size_t first, size_t n)
 {
     if (c->prec == WF_FP64) {
-        WF_TRY_CUDA(cudaMemcpyAsync(dst, src, c->S * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
+        WF_TRY_CUDA(cudaMemcpyAsync((double *)dst + first, src + first, n * sizeof(double), cudaMemcpyDeviceToDevice,
+                                    c->stream));
         return WF_OK;
     }
-    k_to_prec<float><<<592, 256, 0, c->stream>>>((float *)dst, src, c->S);
+    k_to_prec<float><<<592, 256, 0, c->stream>>>((float *)dst + first, src + first, n);
     WF_TRY_CUDA(cudaGetLastError());
     return WF_OK;
 }
+wf_status put_state_dev(wf_ctx *c, void *dst, const double *src) { return put_values_dev(c, dst, src, 0, c->S); }
 
 wf_status get_state_dev(wf_ctx *c, double *dst, const void *src)
 {
@@ -2022,9 +2024,20 @@ wf_status wf_pressure_device(wf_ctx *c, const double *y_np1, const double *y_n, 
     if (!c || !y_np1 || !y_n || !pr) { set_error("wf_pressure_device: null argument"); return WF_ERR_ARG; }
     if (const wf_status st0 = settle_p(c)) return st0;
     void *b1 = c->ybuf[1 - c->cur], *bn = c->Xa ? c->Xa : c->ybuf[c->cur];
-    wf_status st = put_state_dev(c, b1, y_np1);
-    if (st) return st;
-    if ((st = put_state_dev(c, bn, y_n))) return st;
+    wf_status st;
+    if (c->P.variable_density == 0 && c->Xa) {
+        // the constant-density source reads the velocities of y_np1 and nothing of
+        // y_n, so no more is brought into the context (257 x 200 x 64 in FP64: 3 fields
+        // instead of 8, of the 10 copied around a solve); the last value of each
+        // state goes along, so that a pointer the copies refuse is still refused
+        const size_t last = c->S - 1;
+        if ((st = put_values_dev(c, b1, y_np1, 0, 3 * c->N))) return st;
+        if ((st = put_values_dev(c, b1, y_np1, last, 1))) return st;
+        if ((st = put_values_dev(c, bn, y_n, last, 1))) return st;
+    } else {
+        if ((st = put_state_dev(c, b1, y_np1))) return st;
+        if ((st = put_state_dev(c, bn, y_n))) return st;
+    }
     WF_TRY_CUDA(cudaMemcpyAsync(c->p, pr, sizeof(double) * c->N, cudaMemcpyDeviceToDevice, c->stream));
     st = (c->prec == WF_FP64) ? enqueue_pressure<double>(c, b1, bn) : enqueue_pressure<float>(c, b1, bn);
     if (st) return st;
