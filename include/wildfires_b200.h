@@ -166,11 +166,11 @@ wf_status wf_initial_conditions(wf_ctx *ctx);
 wf_status wf_step(wf_ctx *ctx, int nsteps);
 wf_status wf_synchronize(wf_ctx *ctx);
 
-/* Tile shape of the fused stage pass: TI x TJ columns of 8 planes, processed
- * by `threads` threads per block.  The first wf_step of a context picks it:
- * WF_STAGE_TILE=TIxTJ[/threads] in the environment forces one, otherwise each
- * compiled form (FP32: 8x16/512, 8x16/384, 8x8/256; FP64: 8x8/512, 8x8/256) is timed on
- * the context's own grid and state and the fastest is kept.  All forms give
+/* Block form of the stage pass, named TI x TJ / threads (FP32: 8x16/512, 8x16/384,
+ * 8x8/256; FP64: 8x8/512, 8x8/256).  The names select a form; the tile itself (rows
+ * and planes of a block, and how far it walks along x) is fitted to the grid by
+ * a cost rule.  wf_create takes the form that WF_STAGE_TILE=TIxTJ[/threads] names,
+ * else one by precision and grid size; nothing is timed.  All forms give
  * bit-identical results.  wf_set_stage_tile forces a form (threads <= 0: the
  * first with that TI x TJ; call it before stepping; WF_ERR_ARG for a form that
  * is not compiled).  threads may be NULL in wf_stage_tile.  The tiling is a

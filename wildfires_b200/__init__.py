@@ -199,7 +199,7 @@ class Solver:
         return {f: getattr(d, f) for f, _ in WfDiag._fields_}
 
     def stage_tile(self):
-        """(TI, TJ, threads) of the fused stage pass (picked by the first step)."""
+        """(TI, TJ, threads) naming the block form of the stage pass."""
         ti, tj, nt = C.c_int(), C.c_int(), C.c_int()
         check(lib().wf_stage_tile(self._h, C.byref(ti), C.byref(tj), C.byref(nt)), "wf_stage_tile")
         return ti.value, tj.value, nt.value

@@ -1573,7 +1573,7 @@ wf_status wf_pressure(wf_ctx *c, const double *y_np1, const double *y_n, double 
 // One CUDA graph per ensemble step holds every member's step as a branch of
 // its own (the members' streams fork from and join back to one stream), so the
 // GPU runs the members' kernels concurrently and one graph launch replaces
-// 18 launches per member.  Members whose step is not static (ignition source
+// 15 launches per member.  Members whose step is not static (ignition source
 // active) are enqueued eagerly on their own streams instead.
 }  // extern "C"
 
