@@ -397,8 +397,8 @@ __global__ void __launch_bounds__(256, E::kMinBlocks) k_p_rhs_ffty(const Poisson
     const int nslices = nk + 1;                      // f slices + top-plane pressure
     double *Ad = reinterpret_cast<double *>(smem);
     const int total = n1 * 2 * LB;
-    __shared__ DivZ s_w[2 * LB];   // z weights of the block's slices
-    if (threadIdx.x < 2 * LB && 2 * pair0 + threadIdx.x < nk) s_w[threadIdx.x] = div_weights(g.z, 2 * pair0 + threadIdx.x);
+    __shared__ DivZ s_w[2 * LB];   // z weights of the block's slices (with 8- and 16-point transforms 512, more than threads)
+    for (int q = threadIdx.x; q < 2 * LB && 2 * pair0 + q < nk; q += 256) s_w[q] = div_weights(g.z, 2 * pair0 + q);
     __syncthreads();
     if (a.ph.variable_density == 0) {
         // the source is the scaled divergence: SU points per thread at a
