@@ -44,3 +44,42 @@ def test_one_step_matches_oracle_in_every_form(size, method, extra, params_from_
                     for f, (linf, l2) in field_errors(P, y, yo).items():
                         assert l2 <= tol and (prec == "fp32" or linf <= tol), (prec, f, linf, l2)
                 assert np.array_equal(y, first[0]) and np.array_equal(p, first[1]), (prec, flag, form)
+
+
+@pytest.mark.parametrize("size,extra", [((13, 30, 20), {}), ((9, 25, 33), FULL)])
+def test_fuel_that_jumps_across_the_periodic_seam(size, extra, params_from_text):
+    """The planes i = Nx-1 and j = Ny-1 repeat planes 0 in u, v, w and T, but their fuel is
+    their own (an uneven bed need not close on itself): drag, reaction and convective
+    exchange there take it, the SGS inputs that the neighbours read take plane 0's.  Phi
+    against the CPU oracle with burning cells on the seam, in every form; tolerances as above.
+    The oracle's SGS inputs of the seam take the seam's fuel for its neighbours on the seam: a
+    difference of at most nu / T dS / 3d in a velocity's rate (dS what the fuel changes in T's
+    rate, d the least spacing, 1/3 the divergence source's weight)."""
+    from wildfires_b200 import Solver, configs
+    Nx, Ny, Nz = size
+    case = configs.hill(Nx=Nx, Ny=Ny, Nz=Nz, Nt=1, L=60.0, H=0.5 * Nz, jitter=0.2, seed=Nz, Y_h=3.0, **extra)
+    P = params_from_text(configs.param_text(case.params))
+    y0, _ = case.fields(P)
+    r, N, rng = P.rec, Nx * Ny * Nz, np.random.default_rng(5)
+    T, Y = y0[3 * N:4 * N].reshape(size), y0[4 * N:].reshape(Nx, Ny, r.Nz_Y_max)
+    live = (np.arange(Nz) > P.cut_nodes()[..., None]) & (np.arange(Nz) < P.nz_y()[..., None])
+    T[live] = 700.0 + 0.5 * (T[live] - 300.0)
+    T[-1], T[:, -1] = T[0], T[:, 0]
+    Y[:] = np.where(live[:, :, :Y.shape[2]], rng.uniform(0.0, 1.0, Y.shape) * (rng.uniform(size=Y.shape) < 0.8), 0.0)
+    assert live[-1].any() and live[:, -1].any()
+    want = O.phi(P, y0)
+    closed = y0.copy()
+    Yc = closed[4 * N:].reshape(Y.shape)
+    Yc[-1], Yc[:, -1] = Yc[0], Yc[:, 0]
+    dS = np.max(np.abs(O.phi(P, closed) - want)[3 * N:4 * N])
+    sgs = r.mu * (T.max() / r.T_inf) / (r.T_inf * r.rho_inf) * dS / (3 * min(r.dx, r.dy, np.diff(P.z()).min()))
+    for prec, tol in (("fp64", 1e-10), ("fp32", 1e-5)):
+        for form in FORMS[prec]:
+            with Solver(P, prec) as s:
+                s.set_stage_tile(*form)
+                got = s.phi(y0)
+            for q, (f, (linf, l2)) in enumerate(field_errors(P, got, want).items()):
+                k = want[q * N:(q + 1) * N]
+                more = sgs / np.max(np.abs(k)) if f in "uvw" else 0.0
+                assert l2 <= tol + more * np.sqrt(N) * np.max(np.abs(k)) / np.linalg.norm(k), (prec, form, f, linf, l2)
+                assert prec == "fp32" or linf <= tol + more, (prec, form, f, linf, l2)

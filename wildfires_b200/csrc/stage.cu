@@ -965,6 +965,11 @@ __global__ void __launch_bounds__(NT + FR, NB)
 // column's fuel top never change and are not read, so only the stage that makes
 // the new state copies them.  The thread of the cut node's T also takes the next
 // stage's wall friction velocity, which saves that stage its k_utau.
+// The last planes in x and y repeat the first ones, but for the fuel: the fused
+// pass takes the first planes' for both, and what a seam cell's own fuel changes in
+// its drag, reaction and convective exchange is added here (inside the fused
+// pass the second evaluation spilled 32 to 96 bytes and cost 5% of the FP32 step; here
+// 1 us of a 56 us step of 33 x 33 x 16 in FP64, nothing on the larger grids).
 template <class R>
 __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 12 : 8) k_stage_edge(const StageArgs<R> a, int all_fuel)
 {
@@ -974,6 +979,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 12 : 8) k_stage_edge(con
     if (col >= g.Nx * g.Ny) return;
     const size_t N = (size_t)g.N, cb = (size_t)col * g.Nz;
     const int i = col / g.Ny, wc = wrap_p(i, g.Nx - 1) * g.Ny + wrap_p(col - i * g.Ny, g.Ny - 1);
+    const bool seam = wc != col;
     const int kc = __ldg(g.cut + wc), nzy = __ldg(g.nzy + wc), nf = all_fuel ? g.NzY : nzy;
     const bool rd = stage_reads_acc(a.method, a.stage), kp = stage_keeps_acc(a.method, a.stage);
     const R an = (R)a.a_next;
@@ -984,8 +990,36 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 12 : 8) k_stage_edge(con
     const size_t o = f * N + cb + (top ? g.Nz - 1 : kc);
     const R y = a.yn[o];
     R *bacc = bc + (top ? 11 + f : 10);
+    // whether plane q of a seam column holds other fuel than its copy, and what that adds to the
+    // k-value of field f there
+    auto fuel_jumps = [&](int q) {
+        return seam && q < nzy && a.X[4 * N + (size_t)col * g.NzY + q] != a.X[4 * N + (size_t)wc * g.NzY + q];
+    };
+    auto own_fuel = [&](int q, int f) {
+        const PhysR<R> &r = a.pr;
+        const R Y = a.X[4 * N + (size_t)col * g.NzY + q], Yw = a.X[4 * N + (size_t)wc * g.NzY + q];
+        const R *X = a.X + (size_t)wc * g.Nz + q;
+        if (f < 3) {
+            const R u = X[0], v = X[N], w = X[2 * N];
+            return -r.cd * (Y - Yw) * rsqrt_(u * u + v * v + w * w) * X[f * N];
+        }
+        const R T = X[3 * N], K = r.H_C_cp * (Y - Yw) * arrhenius(r, T);
+        if (r.alpha_s * r.sigma_s == R(0) || (Y > R(0)) == (Yw > R(0))) return K;
+        // the exchange of a cell with fuel less that of one without (sources)
+        const R dz = a.krow[(size_t)q * KROW + RDZ], dT = T - r.T_inf;
+        const R h = r.h_c * dz * rsqrt_(rsqrt_(fdiv(rfabs(dT), dz))) * r.alpha_s * r.sigma_s * dT * r.inv_Trho_cp * (r.T_inf + T);
+        return Y > R(0) ? K + h : K - h;
+    };
+    // added to what is there already: the update is linear in the k-value
+    auto add = [&](size_t at, R *accv, R d) {
+        R dacc = R(0);
+        a.Xout[at] += rk_update(a.method, a.stage, d, R(0), dacc, an);
+        if (kp) *accv += dacc;
+    };
+    const int q1 = top ? g.Nz - 2 : kc + 1, q2 = top ? g.Nz - 3 : kc + 2;   // the cells extrapolated from
+    const bool jumps1 = (top || cutT) && fuel_jumps(q1), jumps2 = (top || cutT) && fuel_jumps(q2);
     R kv = R(0), acc = R(0), T0 = R(1), u[3] = {R(0), R(0), R(0)}, v[3] = {R(0), R(0), R(0)};
-    const bool utau = cutT && a.make_utau;
+    const bool utau = cutT && a.make_utau && !seam;   // of the first planes only, which stand for the last
     if (utau) {
         // for the wall friction velocity: u and v of the cut node keep y_n, the others the
         // fused pass has written
@@ -1004,6 +1038,11 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 12 : 8) k_stage_edge(con
     const R out = rk_update(a.method, a.stage, kv, y, acc, an);
     a.Xout[o] = out;
     if ((top || cutT) && kp) *bacc = acc;
+#pragma unroll 1
+    for (int n = jumps1 ? 0 : 1; n < (jumps2 ? 2 : 1); n++) {
+        const R wt = top ? (n ? -a.pr.top_w2 : a.pr.top_w1) : n ? -w[RCUT2] : w[RCUT1];
+        add(o, bacc, wt * own_fuel(n ? q2 : q1, f));
+    }
     if (utau) a.utau[col] = utau_of(a, u, v, kc == 0 ? out : T0);
     for (int k = p; k < nf; k += 8) {
         // rate -Y_f K(T) Y below the fuel top
@@ -1012,10 +1051,13 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 12 : 8) k_stage_edge(con
             return q < nzy ? -a.pr.Y_f * arrhenius(a.pr, a.X[3 * N + (size_t)wc * g.Nz + q]) * a.X[oY + q - k] : R(0);
         };
         const R yY = a.yn[oY];
+        const bool jumps = k > kc && k < g.Nz - 1 && fuel_jumps(k);
         R aY = (rd && k < nzy) ? a.acc[oY] : R(0), r = R(0);
         if (k < nzy) r = k == kc ? w[RCUT1] * rate(kc + 1) - w[RCUT2] * rate(kc + 2) : k < kc ? a.pr.dead[4] : rate(k);
         a.Xout[oY] = rk_update(a.method, a.stage, r, yY, aY, an);
         if (kp && k < nzy) a.acc[oY] = aY;
+#pragma unroll 1
+        for (int q = 0; jumps && q < 4; q++) add(q * N + cb + k, a.acc + q * N + cb + k, own_fuel(k, q));
     }
 }
 
