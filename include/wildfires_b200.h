@@ -164,6 +164,14 @@ wf_status wf_initial_conditions(wf_ctx *ctx);
  * rules, clamps, temperature source).  Enqueued on the context's stream; the
  * first call records the step into a CUDA graph that later calls replay. */
 wf_status wf_step(wf_ctx *ctx, int nsteps);
+/* Waits for the work enqueued so far.  The stage kernel's waits for the planes of
+ * the state that it loads are bounded (about a second).  When one runs out, the
+ * kernel lets the copies in flight land, raises an error flag and leaves a wrong
+ * state; of the calls that wait for the context (this one, wf_download_state,
+ * wf_diagnostics, wf_timestep_reports, wf_dump_wait, wf_phi, wf_rk,
+ * wf_ensemble_synchronize) the next one returns WF_ERR_CUDA once and clears the
+ * flag.  Calls that only enqueue (wf_step, the device-buffer operators) leave it
+ * to them. */
 wf_status wf_synchronize(wf_ctx *ctx);
 
 /* Block form of the stage pass, named TI x TJ / threads (FP32: 8x16/512, 8x16/384,

@@ -278,7 +278,11 @@ struct wf_ctx {
     double *d_rep = nullptr;        // checkpoint report scratch
     Dumper *dump = nullptr;         // asynchronous dumps (created by the first wf_dump_async)
     int tile = 0;                   // tile shape of the fused stage pass (index)
-    int *d_kerr = nullptr;          // raised by a stage kernel whose bounded wait for a plane gave up
+    // raised by a stage kernel whose bounded wait for a plane gave up: a mapped host word, so that the
+    // entries that synchronise read it without a copy
+    volatile int *kerr = nullptr;
+    int *d_kerr = nullptr;          // its device address
+    int plane_wait = kPlaneWaitLimit;
     // tiling of the fused pass for form plan_tile, and TMA tensor maps (CUtensorMap,
     // 128 bytes) of the buffers a stage reads for the boxes of its tiles and rows
     int plan_tile = -1;
@@ -315,6 +319,17 @@ wf_status settle_p(wf_ctx *c)
         c->p_pending = false;
     }
     return WF_OK;
+}
+
+// After a synchronisation of the context's stream: whether a stage kernel that has run
+// gave up its wait for a plane, so that the state is wrong.  Reported once: the flag is
+// cleared, so that later calls start clean.
+wf_status stage_error(wf_ctx *c, const char *who)
+{
+    if (!*c->kerr) return WF_OK;
+    *c->kerr = 0;
+    set_error("%s: a stage kernel's wait for a state plane timed out", who);
+    return WF_ERR_CUDA;
 }
 
 // Kernel launches of one step: k_utau, per stage the optional closure inference,
@@ -599,6 +614,7 @@ template <class R> StageArgs<R> stage_args(wf_ctx *c, const void *X, const void 
     a.make_utau = c->method != 3 && stage < c->nstages;
     a.tile = c->tile;
     a.kerr = c->d_kerr;
+    a.plane_wait = c->plane_wait;
     if (c->plan_tile != c->tile) plan_stage(c);
     a.grid = c->grid;
     a.tmap[0] = a.tmap[1] = nullptr;
@@ -1124,9 +1140,14 @@ wf_status wf_create(const Parameters *P, int precision, wf_ctx **out)
     e = cudaMemsetAsync(c->p, 0, sizeof(double) * c->N, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) { set_error("wf_create: %s", cudaGetErrorString(e)); return fail(WF_ERR_CUDA); }
-    if ((st = dev_alloc(c, (void **)&c->d_kerr, sizeof(int)))) return fail(st);
-    e = cudaMemset(c->d_kerr, 0, sizeof(int));
-    if (e != cudaSuccess) { set_error("wf_create: %s", cudaGetErrorString(e)); return fail(WF_ERR_CUDA); }
+    if (cudaHostAlloc((void **)&c->kerr, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void **)&c->d_kerr, (void *)c->kerr, 0) != cudaSuccess) {
+        cudaGetLastError();
+        set_error("wf_create: out of host memory");
+        return fail(WF_ERR_OOM);
+    }
+    *c->kerr = 0;
+    if (const char *env = getenv("WF_STAGE_WAIT")) c->plane_wait = std::max(atoi(env), 0);   // polls, to exercise the path
     if (!(getenv("WF_NO_TMA") && atoi(getenv("WF_NO_TMA")))) {
         // for the tensor maps; without it the stage kernel copies its planes by cp.async
         cudaDriverEntryPointQueryResult q;
@@ -1149,6 +1170,7 @@ wf_status wf_destroy(wf_ctx *c)
     for (auto &pl : c->ploop)
         if (pl.ge) cudaGraphExecDestroy(pl.ge);
     for (auto &b : c->bufs) cudaFree(b.p);
+    if (c->kerr) cudaFreeHost((void *)c->kerr);
     if (c->up) cudaStreamSynchronize(c->up);
     if (c->ev_y) cudaEventDestroy(c->ev_y);
     if (c->ev_p) cudaEventDestroy(c->ev_p);
@@ -1232,6 +1254,32 @@ wf_status wf_initial_conditions(wf_ctx *c)
 }  // extern "C"
 
 namespace wfs {
+// Diagnostics of the current state (waits for them).
+wf_status diagnose(wf_ctx *c, wf_diag *out)
+{
+    cudaError_t e = (c->prec == WF_FP64)
+                        ? launch_diag<double>(c->geom, c->ph, (const double *)c->ybuf[c->cur], nullptr, c->d_diag, c->stream)
+                        : launch_diag<float>(c->geom, c->ph, (const float *)c->ybuf[c->cur], nullptr, c->d_diag, c->stream);
+    if (e != cudaSuccess) { set_error("wf_diagnostics: %s", cudaGetErrorString(e)); return WF_ERR_CUDA; }
+    double h[13];
+    WF_TRY_CUDA(cudaMemcpyAsync(h, c->d_diag, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+    WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
+    out->mass = h[0];
+    out->energy = h[1];
+    out->fuel = h[2];
+    out->fuel_consumed = c->fuel0 - h[2];
+    out->max_abs_u = h[4];
+    out->max_abs_v = h[5];
+    out->max_abs_w = h[6];
+    out->T_min = -h[7];
+    out->T_max = h[8];
+    out->Y_min = -h[9];
+    out->Y_max = h[10];
+    out->nan_count = (long long)h[12];
+    out->cfl = c->P.dt * (h[4] / c->P.dx + h[5] / c->P.dy + h[6] / c->P.dz);
+    return out->nan_count ? WF_ERR_NAN : WF_OK;
+}
+
 // After a new initial state: the held temperature source, then the fuel
 // integral the diagnostics report consumption against.
 wf_status finish_upload(wf_ctx *c)
@@ -1243,7 +1291,7 @@ wf_status finish_upload(wf_ctx *c)
     }
     WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
     wf_diag d;
-    const wf_status st = wf_diagnostics(c, &d);
+    const wf_status st = diagnose(c, &d);
     c->fuel0 = d.fuel;
     return st == WF_ERR_NAN ? WF_OK : st;
 }
@@ -1289,7 +1337,7 @@ wf_status wf_download_state(wf_ctx *c, double *y, double *pr)
     if (st) return st;
     WF_TRY_CUDA(cudaMemcpyAsync(pr, c->p, sizeof(double) * c->N, cudaMemcpyDeviceToHost, c->stream));
     WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
-    return WF_OK;
+    return stage_error(c, "wf_download_state");
 }
 
 wf_status wf_step(wf_ctx *c, int nsteps)
@@ -1341,15 +1389,7 @@ wf_status wf_synchronize(wf_ctx *c)
     if (!c) return WF_ERR_ARG;
     if (const wf_status st0 = settle_p(c)) return st0;
     WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
-    if (c->d_kerr) {
-        int herr = 0;
-        WF_TRY_CUDA(cudaMemcpy(&herr, c->d_kerr, sizeof(int), cudaMemcpyDeviceToHost));
-        if (herr) {
-            WF_TRY_CUDA(cudaMemset(c->d_kerr, 0, sizeof(int)));
-            set_error("wf_synchronize: a stage kernel's wait for a state plane timed out");
-            return WF_ERR_CUDA;
-        }
-    }
+    if (const wf_status st = stage_error(c, "wf_synchronize")) return st;
     if (c->closure && c->d_closure_err) {
         int herr = 0;
         WF_TRY_CUDA(cudaMemcpy(&herr, c->d_closure_err, sizeof(int), cudaMemcpyDeviceToHost));
@@ -1401,7 +1441,7 @@ wf_status wf_timestep_reports(wf_ctx *c, wf_report *out)
         out->nan_j = (int)((cell / c->Nz) % (unsigned long long)c->Ny);
         out->nan_i = (int)(cell / ((unsigned long long)c->Nz * c->Ny));
     }
-    return WF_OK;
+    return stage_error(c, "wf_timestep_reports");
 }
 
 wf_status wf_stage_tile(const wf_ctx *c, int *ti, int *tj, int *threads)
@@ -1441,34 +1481,16 @@ wf_status wf_dump_async(wf_ctx *c, const char *dir, int n)
 wf_status wf_dump_wait(wf_ctx *c)
 {
     if (!c) { set_error("wf_dump_wait: null context"); return WF_ERR_ARG; }
-    return dumper_wait(c->dump);
+    const wf_status st = dumper_wait(c->dump);
+    return st ? st : stage_error(c, "wf_dump_wait");
 }
 
 wf_status wf_diagnostics(wf_ctx *c, wf_diag *out)
 {
     const NvtxRange range("wf_diagnostics");
     if (!c || !out) return WF_ERR_ARG;
-    cudaError_t e = (c->prec == WF_FP64)
-                        ? launch_diag<double>(c->geom, c->ph, (const double *)c->ybuf[c->cur], nullptr, c->d_diag, c->stream)
-                        : launch_diag<float>(c->geom, c->ph, (const float *)c->ybuf[c->cur], nullptr, c->d_diag, c->stream);
-    if (e != cudaSuccess) { set_error("wf_diagnostics: %s", cudaGetErrorString(e)); return WF_ERR_CUDA; }
-    double h[13];
-    WF_TRY_CUDA(cudaMemcpyAsync(h, c->d_diag, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-    WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
-    out->mass = h[0];
-    out->energy = h[1];
-    out->fuel = h[2];
-    out->fuel_consumed = c->fuel0 - h[2];
-    out->max_abs_u = h[4];
-    out->max_abs_v = h[5];
-    out->max_abs_w = h[6];
-    out->T_min = -h[7];
-    out->T_max = h[8];
-    out->Y_min = -h[9];
-    out->Y_max = h[10];
-    out->nan_count = (long long)h[12];
-    out->cfl = c->P.dt * (h[4] / c->P.dx + h[5] / c->P.dy + h[6] / c->P.dz);
-    return out->nan_count ? WF_ERR_NAN : WF_OK;
+    const wf_status st = diagnose(c, out), lost = st == WF_OK || st == WF_ERR_NAN ? stage_error(c, "wf_diagnostics") : WF_OK;
+    return lost ? lost : st;
 }
 
 wf_status wf_device_state(wf_ctx *c, void **y, double **pr)
@@ -1545,7 +1567,7 @@ wf_status wf_phi(wf_ctx *c, const double *R_old, double *R_new)
     for (int col = 0; col < c->Nx * c->Ny; col++)
         for (int k = c->hnzy[col]; k < c->NzY; k++) R_new[(size_t)4 * c->N + (size_t)col * c->NzY + k] = 0.0;
     drop_graphs(c);
-    return WF_OK;
+    return stage_error(c, "wf_phi");
 }
 
 wf_status wf_pressure(wf_ctx *c, const double *y_np1, const double *y_n, double *pr, int *iters)
@@ -1718,7 +1740,10 @@ wf_status wf_ensemble_synchronize(wf_ensemble *e)
     if (!e) return WF_ERR_ARG;
     WF_TRY_CUDA(cudaStreamSynchronize(e->master));
     for (wf_ctx *c : e->m) WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
-    return WF_OK;
+    wf_status st = WF_OK;
+    for (wf_ctx *c : e->m)
+        if (const wf_status sc = stage_error(c, "wf_ensemble_synchronize")) st = sc;   // each member's flag is cleared
+    return st;
 }
 
 // ---- learned closure --------------------------------------------------------
@@ -2056,7 +2081,7 @@ wf_status wf_rk(wf_ctx *c, const double *y_n, double *y_np1)
     if (st) return st;
     if ((st = get_state(c, y_np1, y1))) return st;
     drop_graphs(c);
-    return WF_OK;
+    return stage_error(c, "wf_rk");
 }
 
 }  // extern "C"

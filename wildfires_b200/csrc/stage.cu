@@ -191,7 +191,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int lim
     }
     return false;
 }
-constexpr int kTmaWaitLimit = 1 << 20;   // polls before a plane is given up (about a second)
 
 // SGS inputs of a thread's cells
 template <class V> struct Sgs { V mu, g7, S11, S12, S13, S22, S23, S33; };
@@ -561,25 +560,28 @@ __global__ void __launch_bounds__(NT + FR, NB)
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    int lost = -1;   // slot whose plane did not arrive in time: flagged, no further fetches and waits
+    int lost = -1;   // slot whose plane did not arrive in time (+ 8 in the walk): flagged, no further fetches and waits
     auto fetch = [&](int c, int slot) {
         if (!tma) fetch_copy(c, slot);
         else if (lost < 0) fetch_box(c, slot);
     };
     uint32_t phases = 0;
-    auto arrived = [&](int slot) {
+    auto arrived = [&](int slot, int walk) {
         if (tma && lost < 0) {
-            if (mbar_wait(sbase + sm.bar + slot * 8, (phases >> slot) & 1, kTmaWaitLimit)) {
+            if (mbar_wait(sbase + sm.bar + slot * 8, (phases >> slot) & 1, a.plane_wait)) {
                 phases ^= 1u << slot;
             } else {
-                lost = slot;
-                if (a.kerr) atomicExch(a.kerr, 1);
+                lost = slot + walk;
+                if (a.kerr) *(volatile int *)a.kerr = 1;
             }
         }
     };
-    // a late plane gets a bounded chance to land before the block gives up its shared memory
+    // the thread that fetches gives the planes still due a bounded chance to land before the block gives up
+    // its shared memory: of the first four those not waited for, in the walk the one
     auto settle = [&]() {
-        if (lost >= 0) mbar_wait(sbase + sm.bar + lost * 8, (phases >> lost) & 1, kTmaWaitLimit);
+        if (lost >= 0 && issuer)
+            for (int r = lost & 7; r <= (lost < 8 ? 3 : lost & 7); r++)
+                mbar_wait(sbase + sm.bar + r * 8, (phases >> r) & 1, kPlaneWaitLimit);
     };
     for (int c = ib - 2; c <= ib + 1; c++) fetch(c, c - (ib - 2));
 
@@ -591,7 +593,7 @@ __global__ void __launch_bounds__(NT + FR, NB)
         for (int n = 0; n < 3; n++) put_col(ib - 2 + n, h - 1, q[n]);
     }
     if (!tma) asm volatile("cp.async.wait_group 0;" ::: "memory");
-    for (int r = 0; r < 4; r++) arrived(r);
+    for (int r = 0; r < 4; r++) arrived(r, 0);
     block_sync();
     V Y = fuel_at(ib - 1), coef = coef_at(ib - 1);
 
@@ -630,7 +632,7 @@ __global__ void __launch_bounds__(NT + FR, NB)
     auto next_plane = [&](int c) {
         // the plane fetched in this iteration (c + 3) is used from the next one on
         if (!tma) asm volatile("cp.async.wait_group 0;" ::: "memory");
-        if (c + 3 <= ie + 1) arrived(rn);
+        if (c + 3 <= ie + 1) arrived(rn, 8);
         rn = rn == SM::RS - 1 ? 0 : rn + 1;
         am2 = am1;
         am1 = a0;
@@ -711,6 +713,7 @@ __global__ void __launch_bounds__(NT + FR, NB)
             coef = coefn;
             next_plane(c);
         }
+        settle();
     } else {
         // ---- the tile ----
         const bool act = in && gj < Ny && gk < Nz;                  // holds cells of the grid
@@ -952,7 +955,6 @@ __global__ void __launch_bounds__(NT + FR, NB)
             next_plane(c);
         }
     }
-    settle();
 }
 
 // ---------------------------------------------------------------------------

@@ -142,8 +142,10 @@ struct StageArgs {
     StageGrid grid;        // tiling of the grid for that form
     // host copies of the TMA tensor maps (CUtensorMap) of X, by tiles and by rows; nullptr: planes copied by cp.async
     const void *tmap[2];
-    int *kerr;             // set by a stage kernel whose bounded wait for a plane gave up
+    int *kerr;             // host word set by a stage kernel whose bounded wait for a plane gave up
+    int plane_wait;        // polls of each wait for a plane
 };
+constexpr int kPlaneWaitLimit = 1 << 20;   // polls before a plane is given up (about a second)
 
 // Learned closure (closure.cu).
 int closure_param_count();
