@@ -46,6 +46,25 @@ def test_one_step_matches_oracle_in_every_form(size, method, extra, params_from_
                 assert np.array_equal(y, first[0]) and np.array_equal(p, first[1]), (prec, flag, form)
 
 
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_long_walks_refill_the_planes_whose_walls_were_written(prec, params_from_text, monkeypatch):
+    """Walks of more planes than the ring holds (260 x 130 x 24: ten and more), both walls in each tile:
+    the values written beyond the walls of a plane, then the TMA box that takes its place, against
+    copies that know no other way of writing.  Same bits."""
+    from wildfires_b200 import Solver, configs
+    case = configs.hill(Nx=260, Ny=130, Nz=24, Nt=1, L=200.0, H=12.0, jitter=0.2, seed=3)
+    P = params_from_text(configs.param_text(case.params))
+    y0, p0 = case.fields(P)
+    out = []
+    for flag in ("0", "1"):
+        monkeypatch.setenv("WF_NO_TMA", flag)
+        with Solver(P, prec) as s:
+            s.upload(y0, p0)
+            s.step(2)
+            out.append(s.download())
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
 @pytest.mark.parametrize("size,extra", [((13, 30, 20), {}), ((9, 25, 33), FULL)])
 def test_fuel_that_jumps_across_the_periodic_seam(size, extra, params_from_text):
     """The planes i = Nx-1 and j = Ny-1 repeat planes 0 in u, v, w and T, but their fuel is

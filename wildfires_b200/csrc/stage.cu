@@ -72,9 +72,10 @@ __global__ void __launch_bounds__(128) k_utau(const StageArgs<R> a)
 //      c-2, c-1 and c, and the RK update.
 // The fuel and the boundary cells (cut node, top) are k_stage_edge's; what
 // part B writes there is lost, and it leaves the k-values they need in a.bc.
-// State planes arrive three iterations ahead by TMA, one box per plane (one per
-// row where the tile's halo wraps around in y; in x the wrap is the choice of a
-// coordinate);
+// In iteration c plane c + 3 is fetched, and waited for at its end: it is read from
+// iteration c + 1 on, so a load has one iteration to arrive in.  It comes by TMA, one
+// box per plane (one per row where the tile's halo wraps around in y; in x the wrap is
+// the choice of a coordinate);
 // grids whose columns are no multiple of 16 bytes are copied by cp.async instead.
 // One barrier per plane.  FR further threads own the one-cell frame around the
 // tile, whose SGS inputs part B of the tile's edge reads.
@@ -619,6 +620,9 @@ __global__ void __launch_bounds__(NT + FR, NB)
             const R T0 = sh<const R>(oT);   // the weights' sum is zero
             sh<R>(d + e * E) = W(4) * (sh<const R>(oT + st) - T0) + W(5) * (sh<const R>(oT + 2 * st) - T0) + W(6) * (sh<const R>(oT + 3 * st) - T0);
         }
+        // these bytes belong to a TMA box: ordered before the copy that refills the slot (the barriers
+        // between order the threads, not the two ways of writing)
+        if (tma && (has_bot || has_top)) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     };
     if (frame) walls(ib - 1, sm.planeS);
     block_sync();
