@@ -1124,12 +1124,18 @@ template <class R> size_t stage_bytes(int tk, int tj) { return tk > kTileK2 ? St
 
 // Tiling of a grid for blocks of form F on sms multiprocessors: rows per tile and
 // x-planes per block of least cost.  A block takes L + 3 iterations (the two
-// planes around its own, and the first loads); blocks differ (those next to the
-// terrain or the top do more), so several passes of short blocks balance better
-// than one of long ones.  An iteration of a partly filled tile is shorter, but by
-// less than its share of the threads.  A grid that does not fill the machine is
-// charged for part of what it takes of it: short blocks repeat the planes around
-// them, and the rest is there for other members or contexts.
+// planes around its own, and the first loads); an iteration of a partly filled tile is
+// shorter, but by far less than its share of the threads (latency).  Where the blocks
+// fill the machine, passes of short blocks balance better than one of long ones
+// (those next to the terrain or the top do more), hence the quarter pass.  Where they
+// do not, the cost is two fifths the time of a block and three fifths the share of the
+// machine it takes: the first is what a call alone waits for, the second what
+// other contexts and ensemble members lose.  The weights are those of least loss over
+// 8 FP64 and 6 FP32 grids of 17 x 17 x 12 to 128 x 128 x 64, 30 tilings each, timed
+// alone and by three contexts in turn.  Per step, alone / in turn (us), the tilings
+// these weights choose against those of weights that favour small tiles (0.4 + 0.6 of
+// the fill, half and half): 33 x 33 x 16 FP64 135 / 53 (132 / 58), 48 x 40 x 20 FP64 with
+// all source terms 165 / 78 (164 / 92), 64 x 64 x 32 FP32 146 / 67 (139 / 78).
 template <class R, class F> StageGrid plan_form(int Nx, int Ny, int Nz, int sms)
 {
     constexpr int VW = Vec<R>::W;
@@ -1145,13 +1151,13 @@ template <class R, class F> StageGrid plan_form(int Nx, int Ny, int Nz, int sms)
     for (int n = (Ny + jmax - 1) / jmax; n <= Ny; n++) {
         const int tj = (Ny + n - 1) / n;
         if ((Ny + tj - 1) / tj != n) continue;
-        const double iter = 0.4 + 0.6 * (double)(tj * (s.tk / VW)) / F::NT;
+        const double iter = 0.6 + 0.4 * (double)(tj * (s.tk / VW)) / F::NT;
         for (int m = 1; m <= Nx; m++) {
             const int L = (Nx + m - 1) / m;
             if ((Nx + L - 1) / L != m) continue;
             const long long blocks = (long long)s.ntk * n * m, slots = (long long)F::NB * sms;
             const double waves = (double)((blocks + slots - 1) / slots);
-            const double cost = (blocks < slots ? 0.6 + 0.65 * (double)blocks / slots : waves + 0.25) * (L + 3) * iter;
+            const double cost = (blocks < slots ? 0.5 + 0.75 * (double)blocks / slots : waves + 0.25) * (L + 3) * iter;
             if (s.L == 0 || cost < best) {
                 best = cost;
                 s.L = L;
@@ -1299,11 +1305,13 @@ bool stage_tensor_map(void *out, const void *X, int precision, int Nx, int Ny, i
     return r == CUDA_SUCCESS;
 }
 
-// Measured at 512 x 512 x 128 FP32 (ms per launch): 1.19 / 1.25 / 1.11; FP64 at
-// 256 x 256 x 128 0.69 / 0.86, at 201 x 150 x 45 0.22 / 0.26, at 33 x 33 x 16 0.021 / 0.019
-// (blocks of 512 threads hold a whole multiprocessor each, however few of their
-// threads a small grid uses).
-int stage_default_form(int precision, long long cells) { return precision == 0 ? (cells < 200000 ? 1 : 0) : 2; }
+// Measured at 512 x 512 x 128 FP32 (ms per launch): 1.19 / 1.25 / 1.11.  FP64, whole
+// steps alone / by three contexts in turn (us), first form against second: 256 x 256 x 128
+// 0.69 / 0.86 ms per launch, 64 x 64 x 32 201 / 99 against 178 / 112, 64 x 48 x 50 211 / 135
+// against 235 / 157, 100 x 20 x 30 (60,000 cells) equal, 33 x 33 x 16 139 / 54 against 135 / 53,
+// 24 x 24 x 24 129 / 48 against 116 / 46 (a block of 512 threads holds a whole
+// multiprocessor, however few of them a small grid uses).
+int stage_default_form(int precision, long long cells) { return precision == 0 ? (cells < 100000 ? 1 : 0) : 2; }
 int stage_tile_count(int precision) { return precision == 0 ? StageForms<double>::count : StageForms<float>::count; }
 void stage_tile_shape(int precision, int idx, int *ti, int *tj, int *nt)
 {
