@@ -31,6 +31,31 @@ namespace wf {
 
 namespace {
 
+// The kernels of a stage start while the one before them still runs (programmatic
+// dependent launch) and read or write nothing that it touches before after_previous(),
+// which waits for all of it: launch latency, the weights and the index loads are off
+// the chain of a step.  k_stage_march lets the next kernel start in the last iteration of
+// its walk (from its first one on, waiting blocks took the place of other contexts':
+// 33 x 33 x 16 FP64 63 us a step with three contexts in turn against 49; 52 without
+// early starts), the two small kernels at once.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+cudaError_t launch_early(void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t s, A... args)
+{
+    cudaLaunchAttribute early;
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(blocks);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &early;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // ---------------------------------------------------------------------------
 // wall friction velocity of every column from its k = 0 plane
 // (pde.cu:767-772: tau_w = sqrt((mu uz)^2 + (mu vz)^2), u_tau = sqrt(tau_w/rho))
@@ -53,6 +78,7 @@ __global__ void __launch_bounds__(128) k_utau(const StageArgs<R> a)
 {
     const Geom &g = a.g;
     const int col = blockIdx.x * blockDim.x + threadIdx.x;
+    start_next();
     if (col >= g.Nx * g.Ny) return;
     const int Nz = g.Nz, N = g.N;
     const R *X = a.X + (size_t)col * Nz;
@@ -419,6 +445,7 @@ __global__ void __launch_bounds__(NT + FR, NB)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (tma) block_sync();
+    after_previous();   // the weights and the barriers above need nothing of it
     // by TMA, issued by one lane of the block's last warp: a box of the tile's rows,
     // or one per row where the tile's halo wraps around in y
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // uniform in a warp
@@ -660,6 +687,7 @@ __global__ void __launch_bounds__(NT + FR, NB)
         for (int c = ib - 1; c <= ie; c++) {
             if (c + 3 <= ie + 1) fetch(c + 3, rn);
             if (c + 1 < ie) prefetch_rk(c + 1);
+            if (c == ie) start_next();
             V Yn = c_(R(0)), coefn = c_(R(1));
             Col col = {};
             if (c < ie) {
@@ -992,6 +1020,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 12 : 8) k_stage_edge(con
     const int i = col / g.Ny, wc = wrap_p(i, g.Nx - 1) * g.Ny + wrap_p(col - i * g.Ny, g.Ny - 1);
     const bool seam = wc != col;
     const int kc = __ldg(g.cut + wc), nzy = __ldg(g.nzy + wc), nf = all_fuel ? g.NzY : nzy;
+    start_next();
+    after_previous();
     const bool rd = stage_reads_acc(a.method, a.stage), kp = stage_keeps_acc(a.method, a.stage);
     const R an = (R)a.a_next;
     R *bc = a.bc + (size_t)col * kBcSlots;
@@ -1252,26 +1282,23 @@ template <class R> cudaError_t launch_stage(const StageArgs<R> &a, cudaStream_t 
         const int blocks = sg.ntk * sg.ntj * sg.nti, threads = F::NT + F::FR;
         const size_t smem = stage_bytes<R>(sg.tk, sg.tj);
         auto go = [&](auto kw, auto lean_, auto vec_) {
-            k_stage_march<R, F::NT, F::FR, F::NB, decltype(kw)::value, decltype(lean_)::value, decltype(vec_)::value>
-                <<<blocks, threads, smem, s>>>(a, cv, sg, m[0], m[1]);
+            return launch_early(k_stage_march<R, F::NT, F::FR, F::NB, decltype(kw)::value, decltype(lean_)::value, decltype(vec_)::value>,
+                                blocks, threads, smem, s, a, cv, sg, m[0], m[1]);
         };
         auto go_kw = [&](auto kw) {
             if (Vec<R>::W == 1 || a.g.Nz % Vec<R>::W == 0) {   // a thread's cells are one aligned access
-                if (lean) go(kw, std::true_type(), std::true_type());
-                else go(kw, std::false_type(), std::true_type());
+                return lean ? go(kw, std::true_type(), std::true_type()) : go(kw, std::false_type(), std::true_type());
             } else if constexpr (Vec<R>::W > 1) {
-                if (lean) go(kw, std::true_type(), std::false_type());
-                else go(kw, std::false_type(), std::false_type());
+                return lean ? go(kw, std::true_type(), std::false_type()) : go(kw, std::false_type(), std::false_type());
             }
+            return cudaErrorInvalidValue;
         };
-        if (sg.tk > kTileK2) go_kw(std::integral_constant<int, kTileK>());
-        else go_kw(std::integral_constant<int, kTileK2>());
-        return cudaSuccess;
+        return sg.tk > kTileK2 ? go_kw(std::integral_constant<int, kTileK>()) : go_kw(std::integral_constant<int, kTileK2>());
     });
     if (e) return e;
     if (ev) cudaEventRecord(ev[1], s);
     const bool last = a.method == 3 || !stage_keeps_acc(a.method, a.stage);
-    k_stage_edge<R><<<(unsigned)((8 * (size_t)ncol + 127) / 128), 128, 0, s>>>(a, last);
+    if ((e = launch_early(k_stage_edge<R>, (unsigned)((8 * (size_t)ncol + 127) / 128), 128, 0, s, a, (int)last))) return e;
     if (ev) cudaEventRecord(ev[2], s);
     return cudaGetLastError();
 }
