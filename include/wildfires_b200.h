@@ -168,10 +168,10 @@ wf_status wf_step(wf_ctx *ctx, int nsteps);
  * the state that it loads are bounded (about a second).  When one runs out, the
  * kernel lets the copies in flight land, raises an error flag and leaves a wrong
  * state; of the calls that wait for the context (this one, wf_download_state,
- * wf_diagnostics, wf_timestep_reports, wf_dump_wait, wf_phi, wf_rk,
+ * wf_diagnostics, wf_timestep_reports, wf_phi, wf_rk,
  * wf_ensemble_synchronize) the next one returns WF_ERR_CUDA once and clears the
- * flag.  Calls that only enqueue (wf_step, the device-buffer operators) leave it
- * to them. */
+ * flag.  Calls that only enqueue (wf_step, the device-buffer operators, dumps) leave
+ * it to them. */
 wf_status wf_synchronize(wf_ctx *ctx);
 
 /* Block form of the stage pass, named TI x TJ / threads (FP32: 8x16/512, 8x16/384,

@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(kRepThreads) k_report_part(const Geom g, const
 // and the warps in order (maxima and the smallest key: any order gives the
 // same result).
 __global__ void __launch_bounds__(kRepThreads) k_report_final(const RepPart *__restrict__ parts, int n,
-                                                              double *__restrict__ out)
+                                                              double *__restrict__ out, const int *__restrict__ lost)
 {
     double e[7];
 #pragma unroll
@@ -123,26 +123,28 @@ __global__ void __launch_bounds__(kRepThreads) k_report_final(const RepPart *__r
         unsigned long long k = redk[0];
         for (int w = 1; w < kRepThreads / 32; w++) k = min(k, redk[w]);
         reinterpret_cast<unsigned long long *>(out)[7] = k;
+    } else if (threadIdx.x == 8) {
+        reinterpret_cast<long long *>(out)[8] = *lost;
     }
 }
 
 }  // namespace
 
-size_t report_scratch_bytes() { return sizeof(RepPart) * kRepBlocks + 8 * sizeof(double); }
+size_t report_scratch_bytes() { return sizeof(RepPart) * kRepBlocks + 10 * sizeof(double); }
 
 template <class R>
 cudaError_t launch_report(const Geom &g, const R *y, const double *xg, const double *yg, const double rect[4],
-                          double *scratch, cudaStream_t s)
+                          double *scratch, const int *lost, cudaStream_t s)
 {
-    RepPart *parts = reinterpret_cast<RepPart *>(scratch + 8);
+    RepPart *parts = reinterpret_cast<RepPart *>(scratch + 10);
     k_report_part<R><<<kRepBlocks, kRepThreads, 0, s>>>(g, y, xg, yg, make_double4(rect[0], rect[1], rect[2], rect[3]),
                                                          parts);
-    k_report_final<<<1, kRepThreads, 0, s>>>(parts, kRepBlocks, scratch);
+    k_report_final<<<1, kRepThreads, 0, s>>>(parts, kRepBlocks, scratch, lost);
     return cudaGetLastError();
 }
 template cudaError_t launch_report<double>(const Geom &, const double *, const double *, const double *,
-                                           const double *, double *, cudaStream_t);
+                                           const double *, double *, const int *, cudaStream_t);
 template cudaError_t launch_report<float>(const Geom &, const float *, const double *, const double *,
-                                          const double *, double *, cudaStream_t);
+                                          const double *, double *, const int *, cudaStream_t);
 
 }  // namespace wf

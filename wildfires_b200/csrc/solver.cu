@@ -278,10 +278,9 @@ struct wf_ctx {
     double *d_rep = nullptr;        // checkpoint report scratch
     Dumper *dump = nullptr;         // asynchronous dumps (created by the first wf_dump_async)
     int tile = 0;                   // tile shape of the fused stage pass (index)
-    // raised by a stage kernel whose bounded wait for a plane gave up: a mapped host word, so that the
-    // entries that synchronise read it without a copy
-    volatile int *kerr = nullptr;
-    int *d_kerr = nullptr;          // its device address
+    // raised by a stage kernel whose bounded wait for a plane gave up: a word behind the diagnostics (a
+    // mapped host word would cost 2.5 ms a context), for members of an ensemble one of its array
+    int *d_kerr = nullptr;
     int plane_wait = kPlaneWaitLimit;
     // tiling of the fused pass for form plan_tile, and TMA tensor maps (CUtensorMap,
     // 128 bytes) of the buffers a stage reads for the boxes of its tiles and rows
@@ -321,15 +320,23 @@ wf_status settle_p(wf_ctx *c)
     return WF_OK;
 }
 
-// After a synchronisation of the context's stream: whether a stage kernel that has run
-// gave up its wait for a plane, so that the state is wrong.  Reported once: the flag is
-// cleared, so that later calls start clean.
-wf_status stage_error(wf_ctx *c, const char *who)
+// Whether a stage kernel that has run gave up its wait for a plane, so that the state is
+// wrong (waits for the context's stream).  Reported once: the flag is cleared, so that
+// later calls start clean.
+wf_status stage_error(wf_ctx *c, const char *who, int lost)
 {
-    if (!*c->kerr) return WF_OK;
-    *c->kerr = 0;
+    if (!lost) return WF_OK;
+    WF_TRY_CUDA(cudaMemsetAsync(c->d_kerr, 0, sizeof(int), c->stream));
+    WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
     set_error("%s: a stage kernel's wait for a state plane timed out", who);
     return WF_ERR_CUDA;
+}
+wf_status stage_error(wf_ctx *c, const char *who)
+{
+    int lost = 0;
+    WF_TRY_CUDA(cudaMemcpyAsync(&lost, c->d_kerr, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
+    return stage_error(c, who, lost);
 }
 
 // Kernel launches of one step: k_utau, per stage the optional closure inference,
@@ -1140,13 +1147,9 @@ wf_status wf_create(const Parameters *P, int precision, wf_ctx **out)
     e = cudaMemsetAsync(c->p, 0, sizeof(double) * c->N, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) { set_error("wf_create: %s", cudaGetErrorString(e)); return fail(WF_ERR_CUDA); }
-    if (cudaHostAlloc((void **)&c->kerr, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostGetDevicePointer((void **)&c->d_kerr, (void *)c->kerr, 0) != cudaSuccess) {
-        cudaGetLastError();
-        set_error("wf_create: out of host memory");
-        return fail(WF_ERR_OOM);
-    }
-    *c->kerr = 0;
+    c->d_kerr = reinterpret_cast<int *>(c->d_diag + kDiagValues);
+    e = cudaMemset(c->d_kerr, 0, sizeof(int));
+    if (e != cudaSuccess) { set_error("wf_create: %s", cudaGetErrorString(e)); return fail(WF_ERR_CUDA); }
     if (const char *env = getenv("WF_STAGE_WAIT")) c->plane_wait = std::max(atoi(env), 0);   // polls, to exercise the path
     if (!(getenv("WF_NO_TMA") && atoi(getenv("WF_NO_TMA")))) {
         // for the tensor maps; without it the stage kernel copies its planes by cp.async
@@ -1170,7 +1173,6 @@ wf_status wf_destroy(wf_ctx *c)
     for (auto &pl : c->ploop)
         if (pl.ge) cudaGraphExecDestroy(pl.ge);
     for (auto &b : c->bufs) cudaFree(b.p);
-    if (c->kerr) cudaFreeHost((void *)c->kerr);
     if (c->up) cudaStreamSynchronize(c->up);
     if (c->ev_y) cudaEventDestroy(c->ev_y);
     if (c->ev_p) cudaEventDestroy(c->ev_p);
@@ -1254,16 +1256,18 @@ wf_status wf_initial_conditions(wf_ctx *c)
 }  // extern "C"
 
 namespace wfs {
-// Diagnostics of the current state (waits for them).
-wf_status diagnose(wf_ctx *c, wf_diag *out)
+// Diagnostics of the current state (waits for them), and the stage kernels' error flag.
+wf_status diagnose(wf_ctx *c, wf_diag *out, int *lost)
 {
     cudaError_t e = (c->prec == WF_FP64)
                         ? launch_diag<double>(c->geom, c->ph, (const double *)c->ybuf[c->cur], nullptr, c->d_diag, c->stream)
                         : launch_diag<float>(c->geom, c->ph, (const float *)c->ybuf[c->cur], nullptr, c->d_diag, c->stream);
     if (e != cudaSuccess) { set_error("wf_diagnostics: %s", cudaGetErrorString(e)); return WF_ERR_CUDA; }
-    double h[13];
+    double h[kDiagValues + 1];
     WF_TRY_CUDA(cudaMemcpyAsync(h, c->d_diag, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+    if (c->member) WF_TRY_CUDA(cudaMemcpyAsync(&h[kDiagValues], c->d_kerr, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
+    memcpy(lost, &h[kDiagValues], sizeof(int));
     out->mass = h[0];
     out->energy = h[1];
     out->fuel = h[2];
@@ -1291,7 +1295,8 @@ wf_status finish_upload(wf_ctx *c)
     }
     WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
     wf_diag d;
-    const wf_status st = diagnose(c, &d);
+    int lost;   // of a step before: left for the next call that reports it
+    const wf_status st = diagnose(c, &d, &lost);
     c->fuel0 = d.fuel;
     return st == WF_ERR_NAN ? WF_OK : st;
 }
@@ -1335,9 +1340,13 @@ wf_status wf_download_state(wf_ctx *c, double *y, double *pr)
     if (st) return st;
     st = get_state(c, y, c->ybuf[c->cur]);
     if (st) return st;
+    // the flag on a stream of its own (the steps are done), so that its copy runs beside p's
+    int lost = 0;
     WF_TRY_CUDA(cudaMemcpyAsync(pr, c->p, sizeof(double) * c->N, cudaMemcpyDeviceToHost, c->stream));
+    WF_TRY_CUDA(cudaMemcpyAsync(&lost, c->d_kerr, sizeof(int), cudaMemcpyDeviceToHost, c->aux));
     WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
-    return stage_error(c, "wf_download_state");
+    WF_TRY_CUDA(cudaStreamSynchronize(c->aux));
+    return stage_error(c, "wf_download_state", lost);
 }
 
 wf_status wf_step(wf_ctx *c, int nsteps)
@@ -1388,7 +1397,6 @@ wf_status wf_synchronize(wf_ctx *c)
 {
     if (!c) return WF_ERR_ARG;
     if (const wf_status st0 = settle_p(c)) return st0;
-    WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
     if (const wf_status st = stage_error(c, "wf_synchronize")) return st;
     if (c->closure && c->d_closure_err) {
         int herr = 0;
@@ -1418,11 +1426,11 @@ wf_status wf_timestep_reports(wf_ctx *c, wf_report *out)
     const double rect[4] = {c->P.Y0_x_start, c->P.Y0_x_end, c->P.Y0_y_start, c->P.Y0_y_end};
     cudaError_t e = (c->prec == WF_FP64)
                         ? launch_report<double>(c->geom, (const double *)c->ybuf[c->cur], c->d_x, c->d_y, rect, c->d_rep,
-                                                c->stream)
+                                                c->d_kerr, c->stream)
                         : launch_report<float>(c->geom, (const float *)c->ybuf[c->cur], c->d_x, c->d_y, rect, c->d_rep,
-                                               c->stream);
+                                               c->d_kerr, c->stream);
     if (e != cudaSuccess) { set_error("wf_timestep_reports: %s", cudaGetErrorString(e)); return WF_ERR_CUDA; }
-    double h[8];
+    double h[9];
     WF_TRY_CUDA(cudaMemcpyAsync(h, c->d_rep, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
     WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
     // functions.cu:180, same operation order
@@ -1441,7 +1449,9 @@ wf_status wf_timestep_reports(wf_ctx *c, wf_report *out)
         out->nan_j = (int)((cell / c->Nz) % (unsigned long long)c->Ny);
         out->nan_i = (int)(cell / ((unsigned long long)c->Nz * c->Ny));
     }
-    return stage_error(c, "wf_timestep_reports");
+    long long lost;
+    memcpy(&lost, &h[8], sizeof(lost));
+    return stage_error(c, "wf_timestep_reports", (int)lost);
 }
 
 wf_status wf_stage_tile(const wf_ctx *c, int *ti, int *tj, int *threads)
@@ -1481,16 +1491,16 @@ wf_status wf_dump_async(wf_ctx *c, const char *dir, int n)
 wf_status wf_dump_wait(wf_ctx *c)
 {
     if (!c) { set_error("wf_dump_wait: null context"); return WF_ERR_ARG; }
-    const wf_status st = dumper_wait(c->dump);
-    return st ? st : stage_error(c, "wf_dump_wait");
+    return dumper_wait(c->dump);
 }
 
 wf_status wf_diagnostics(wf_ctx *c, wf_diag *out)
 {
     const NvtxRange range("wf_diagnostics");
     if (!c || !out) return WF_ERR_ARG;
-    const wf_status st = diagnose(c, out), lost = st == WF_OK || st == WF_ERR_NAN ? stage_error(c, "wf_diagnostics") : WF_OK;
-    return lost ? lost : st;
+    int lost = 0;
+    const wf_status st = diagnose(c, out, &lost), se = stage_error(c, "wf_diagnostics", lost);
+    return se ? se : st;
 }
 
 wf_status wf_device_state(wf_ctx *c, void **y, double **pr)
@@ -1605,6 +1615,7 @@ struct wf_ensemble {
     cudaEvent_t fork = nullptr;
     std::vector<cudaEvent_t> join;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    int *d_kerr = nullptr;   // the members' error flags, side by side
     int parity = 0;
 };
 
@@ -1664,6 +1675,13 @@ wf_status wf_ensemble_create(const Parameters *members, int n_members, int preci
         }
         e->join.push_back(ev);
     }
+    if (cudaMalloc(&e->d_kerr, sizeof(int) * n_members) != cudaSuccess ||
+        cudaMemset(e->d_kerr, 0, sizeof(int) * n_members) != cudaSuccess) {
+        cudaGetLastError();
+        set_error("wf_ensemble_create: device allocation failed");
+        return fail(WF_ERR_OOM);
+    }
+    for (int i = 0; i < n_members; i++) e->m[i]->d_kerr = e->d_kerr + i;
     *out = e;
     return WF_OK;
 }
@@ -1674,6 +1692,7 @@ wf_status wf_ensemble_destroy(wf_ensemble *e)
     if (e->master) cudaStreamSynchronize(e->master);
     ensemble_drop_graphs(e);
     for (wf_ctx *c : e->m) wf_destroy(c);
+    cudaFree(e->d_kerr);
     for (cudaEvent_t ev : e->join) cudaEventDestroy(ev);
     if (e->fork) cudaEventDestroy(e->fork);
     if (e->master) cudaStreamDestroy(e->master);
@@ -1738,11 +1757,13 @@ wf_status wf_ensemble_step(wf_ensemble *e, int nsteps)
 wf_status wf_ensemble_synchronize(wf_ensemble *e)
 {
     if (!e) return WF_ERR_ARG;
-    WF_TRY_CUDA(cudaStreamSynchronize(e->master));
     for (wf_ctx *c : e->m) WF_TRY_CUDA(cudaStreamSynchronize(c->stream));
+    std::vector<int> lost(e->m.size());
+    WF_TRY_CUDA(cudaMemcpyAsync(lost.data(), e->d_kerr, sizeof(int) * lost.size(), cudaMemcpyDeviceToHost, e->master));
+    WF_TRY_CUDA(cudaStreamSynchronize(e->master));
     wf_status st = WF_OK;
-    for (wf_ctx *c : e->m)
-        if (const wf_status sc = stage_error(c, "wf_ensemble_synchronize")) st = sc;   // each member's flag is cleared
+    for (size_t q = 0; q < lost.size(); q++)
+        if (const wf_status sc = stage_error(e->m[q], "wf_ensemble_synchronize", lost[q])) st = sc;   // each flag is cleared
     return st;
 }
 

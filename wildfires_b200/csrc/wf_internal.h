@@ -142,7 +142,7 @@ struct StageArgs {
     StageGrid grid;        // tiling of the grid for that form
     // host copies of the TMA tensor maps (CUtensorMap) of X, by tiles and by rows; nullptr: planes copied by cp.async
     const void *tmap[2];
-    int *kerr;             // host word set by a stage kernel whose bounded wait for a plane gave up
+    int *kerr;             // set by a stage kernel whose bounded wait for a plane gave up
     int plane_wait;        // polls of each wait for a plane
 };
 constexpr int kPlaneWaitLimit = 1 << 20;   // polls before a plane is given up (about a second)
@@ -250,17 +250,20 @@ constexpr int kMaxFftLength = 2048;     // longest supported x or y transform
 constexpr int kMaxZUnknowns = 511;      // longest tridiagonal system (Nz-1): the projection runs one
                                         // thread per cell of a column, at most 512
 
-// Grid-wide FP64 reductions for the diagnostics and the pressure fixed point.
+// Grid-wide FP64 reductions for the diagnostics and the pressure fixed point: kDiagValues results, of 16
+// places, then scratch.
+constexpr int kDiagValues = 13;
 template <class R>
 cudaError_t launch_diag(const Geom &g, const Phys &ph, const R *y, const R *y0fuel_ref, double *out, cudaStream_t s);
 
 // Reference-style checkpoint report (functions.cu:82-185): scratch[0..6] =
 // max|u|, max|v|, max|w|, -T_min, T_max, -Y_min, Y_max (fuel rectangle for T
-// and Y), scratch[7] = first NaN key ((i Ny + j) Nz + k) * 5 + field as bits, or ~0.
+// and Y), scratch[7] = first NaN key ((i Ny + j) Nz + k) * 5 + field as bits, or ~0,
+// scratch[8] = *lost (the stage kernels' error flag) as an integer.
 size_t report_scratch_bytes();
 template <class R>
 cudaError_t launch_report(const Geom &g, const R *y, const double *xg, const double *yg, const double rect[4],
-                          double *scratch, cudaStream_t s);
+                          double *scratch, const int *lost, cudaStream_t s);
 
 // Initial conditions on the device (setup.cu; functions.cu:187-323).
 struct IcArgs {
