@@ -178,7 +178,9 @@ wf_status wf_synchronize(wf_ctx *ctx);
  * 8x8/256; FP64: 8x8/512, 8x8/256).  The names select a form; the tile itself (rows
  * and planes of a block, and how far it walks along x) is fitted to the grid by
  * a cost rule.  wf_create takes the form that WF_STAGE_TILE=TIxTJ[/threads] names,
- * else one by precision and grid size; nothing is timed.  All forms give
+ * else one by precision and grid size; nothing is timed.  A WF_STAGE_TILE that names
+ * no form leaves that one in place and makes wf_step and wf_ensemble_step return
+ * WF_ERR_ARG until wf_set_stage_tile is called.  All forms give
  * bit-identical results.  wf_set_stage_tile forces a form (threads <= 0: the
  * first with that TI x TJ; call it before stepping; WF_ERR_ARG for a form that
  * is not compiled).  threads may be NULL in wf_stage_tile.  The tiling is a

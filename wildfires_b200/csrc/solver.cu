@@ -277,7 +277,8 @@ struct wf_ctx {
     int closure_wait = kClosureWaitLimit;   // polls of each tensor-core completion wait
     double *d_rep = nullptr;        // checkpoint report scratch
     Dumper *dump = nullptr;         // asynchronous dumps (created by the first wf_dump_async)
-    int tile = 0;                   // tile shape of the fused stage pass (index)
+    int tile = 0;                   // block form of the fused stage pass (index)
+    std::string bad_tile;           // WF_STAGE_TILE at creation, where it names no form: steps are refused
     // raised by a stage kernel whose bounded wait for a plane gave up: a word behind the diagnostics (a
     // mapped host word would cost 2.5 ms a context), for members of an ensemble one of its array
     int *d_kerr = nullptr;
@@ -291,7 +292,6 @@ struct wf_ctx {
         const void *ptr = nullptr;
         alignas(64) unsigned char tile[128], row[128];
     } tmaps[4];
-    bool tile_set = false;          // chosen by choose_tile or wf_set_stage_tile
     // wf_upload_state_async: p is copied on `up` after the state's copy (event
     // ev_y) and completes ev_p; the step waits for ev_p just before its pressure
     // solve, every other user of p first makes the context stream wait for it
@@ -307,7 +307,8 @@ struct wf_ctx {
 namespace wfs {
 
 wf_status finish_upload(wf_ctx *c);
-wf_status choose_tile(wf_ctx *c);
+void choose_tile(wf_ctx *c);
+wf_status tile_error(const wf_ctx *c);
 
 // Order the context stream after a pressure copy of wf_upload_state_async that
 // may still be in flight (callers that read or write p other than the step).
@@ -1159,6 +1160,7 @@ wf_status wf_create(const Parameters *P, int precision, wf_ctx **out)
             c->encode = nullptr;
         cudaGetLastError();
     }
+    choose_tile(c);
     c->launches = launches_per_step(c);
     *out = c;
     return WF_OK;
@@ -1301,32 +1303,34 @@ wf_status finish_upload(wf_ctx *c)
     return st == WF_ERR_NAN ? WF_OK : st;
 }
 
-// Block form of the fused stage pass for this context: WF_STAGE_TILE=TIxTJ[/threads]
+// Block form of the fused stage pass for a new context: WF_STAGE_TILE=TIxTJ[/threads]
 // in the environment forces one, otherwise the one stage_default_form gives for the grid.
 // Every form gives bit-identical results: a cell's arithmetic does not depend
 // on the tiling.
-wf_status choose_tile(wf_ctx *c)
+void choose_tile(wf_ctx *c)
 {
-    if (c->tile_set) return WF_OK;
-    c->tile_set = true;
     const int prec = c->prec == WF_FP64 ? 0 : 1, count = stage_tile_count(prec);
     c->tile = stage_default_form(prec, c->N);
-    if (const char *env = getenv("WF_STAGE_TILE")) {
-        int ti = 0, tj = 0, nt = 0;
-        const int got = sscanf(env, "%dx%d/%d", &ti, &tj, &nt);   // TIxTJ, optionally /threads
-        if (got >= 2)
-            for (int q = 0; q < count; q++) {
-                int a = 0, b = 0, n = 0;
-                stage_tile_shape(prec, q, &a, &b, &n);
-                if (a == ti && b == tj && (got < 3 || n == nt)) {
-                    c->tile = q;
-                    return WF_OK;
-                }
-            }
-        set_error("WF_STAGE_TILE=%s is not a compiled tile shape", env);
-        return WF_ERR_ARG;
+    const char *env = getenv("WF_STAGE_TILE");
+    if (!env) return;
+    int ti = 0, tj = 0, nt = 0;
+    const int got = sscanf(env, "%dx%d/%d", &ti, &tj, &nt);   // TIxTJ, optionally /threads
+    for (int q = 0; got >= 2 && q < count; q++) {
+        int a = 0, b = 0, n = 0;
+        stage_tile_shape(prec, q, &a, &b, &n);
+        if (a == ti && b == tj && (got < 3 || n == nt)) {
+            c->tile = q;
+            return;
+        }
     }
-    return WF_OK;
+    c->bad_tile = *env ? env : "(empty)";
+}
+// Whether the context may step: not while the form it was told to take does not exist.
+wf_status tile_error(const wf_ctx *c)
+{
+    if (c->bad_tile.empty()) return WF_OK;
+    set_error("WF_STAGE_TILE=%s is not a compiled tile shape", c->bad_tile.c_str());
+    return WF_ERR_ARG;
 }
 }  // namespace wfs
 
@@ -1353,10 +1357,8 @@ wf_status wf_step(wf_ctx *c, int nsteps)
 {
     const NvtxRange range("wf_step");
     if (!c || nsteps < 0) { set_error("wf_step: invalid argument"); return WF_ERR_ARG; }
-    if (nsteps > 0) {
-        const wf_status st = choose_tile(c);
-        if (st) return st;
-    }
+    if (nsteps > 0)
+        if (const wf_status st = tile_error(c)) return st;
     for (int q = 0; q < nsteps; q++) {
         const int n1 = c->n + 1;
         if (step_is_static(c, n1)) {
@@ -1470,7 +1472,7 @@ wf_status wf_set_stage_tile(wf_ctx *c, int ti, int tj, int threads)
         stage_tile_shape(prec, q, &a, &b, &n);
         if (a == ti && b == tj && (threads <= 0 || n == threads)) {
             c->tile = q;
-            c->tile_set = true;
+            c->bad_tile.clear();
             drop_graphs(c);
             return WF_OK;
         }
@@ -1716,7 +1718,7 @@ wf_status wf_ensemble_step(wf_ensemble *e, int nsteps)
     const NvtxRange range("wf_ensemble_step");
     if (!e || nsteps < 0) { set_error("wf_ensemble_step: invalid argument"); return WF_ERR_ARG; }
     for (wf_ctx *c : e->m) {
-        const wf_status st = nsteps > 0 ? choose_tile(c) : WF_OK;
+        const wf_status st = nsteps > 0 ? tile_error(c) : WF_OK;
         if (st) return st;
     }
     for (int q = 0; q < nsteps; q++) {
