@@ -698,7 +698,8 @@ constexpr int kThomasAhead = 8;
 constexpr int kThomasThreads = 64;
 constexpr int kThomasMaxPlanes = 256;   // 256 x 8 bytes x 32 systems = 64 KB, three blocks per SM
 
-// v / u with rec = 1 / u
+// v / u with rec = 1 / u.  Where v or rec is infinite this is NaN and the quotient would be
+// infinite or 0; the transform of a source that holds an infinity is NaN throughout anyway.
 __device__ __forceinline__ double quotient(double v, double u, double rec)
 {
     const double q = v * rec;

@@ -13,6 +13,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <string>
 #include <vector>
@@ -2007,7 +2008,7 @@ wf_status put_values_dev(wf_ctx *c, void *dst, const double *src, size_t first, 
                                     c->stream));
         return WF_OK;
     }
-    k_to_prec<float><<<592, 256, 0, c->stream>>>((float *)dst + first, src + first, n);
+    k_to_prec<float><<<(unsigned)std::min<size_t>(592, (n + 255) / 256), 256, 0, c->stream>>>((float *)dst + first, src + first, n);
     WF_TRY_CUDA(cudaGetLastError());
     return WF_OK;
 }
@@ -2076,8 +2077,11 @@ wf_status wf_pressure_device(wf_ctx *c, const double *y_np1, const double *y_n, 
     if (c->P.variable_density == 0 && c->Xa) {
         // the constant-density source reads the velocities of y_np1 and nothing of
         // y_n, so no more is brought into the context (257 x 200 x 64 in FP64: 3 fields
-        // instead of 8, of the 10 copied around a solve); the last value of each
-        // state goes along, so that a pointer the copies refuse is still refused
+        // instead of 8, of the 10 copied around a solve).  The last value of each state
+        // goes along: an FP64 copy refuses a pointer or an extent that is not the
+        // caller's, and FP32's conversion reads what it always read.  Contexts without Xa
+        // (Euler) take y_n into their current state, which a download then returns: there
+        // both states come whole.
         const size_t last = c->S - 1;
         if ((st = put_values_dev(c, b1, y_np1, 0, 3 * c->N))) return st;
         if ((st = put_values_dev(c, b1, y_np1, last, 1))) return st;

@@ -106,7 +106,11 @@ __global__ void __launch_bounds__(128) k_utau(const StageArgs<R> a)
 // One barrier per plane.  FR further threads own the one-cell frame around the
 // tile, whose SGS inputs part B of the tile's edge reads.
 constexpr int kColRing = 8;   // x-planes of column tables kept (power of two)
-constexpr int kTileK = 32, kTileK2 = 24;   // planes of a tile at most: the two row lengths compiled
+// Planes of a tile at most: the two row lengths compiled.  Rows of 24 leave shared memory for more rows
+// per tile where a column divides into so few planes (step, us, three contexts in turn, against rows of
+// 32 alone: 33 x 33 x 16 FP64 50 / 57, 100 x 100 x 24 FP64 175 / 199, 201 x 150 x 45 FP32 with all source
+// terms 366 / 408, 160 x 128 x 48 FP32 316 / 322).
+constexpr int kTileK = 32, kTileK2 = 24;
 
 // value of a thread's VW cells
 struct F2 {
