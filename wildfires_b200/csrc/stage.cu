@@ -653,13 +653,18 @@ __global__ void __launch_bounds__(NT + FR, NB)
         }
     };
     // The bytes that walls() writes belong to a TMA box: ordered before the copy that refills the slot (the
-    // barriers between order the threads, not the two ways of writing).  At the end of an iteration: right
-    // after the writes the fence waited for the loads in flight (256 x 256 x 128 FP64 3.35 ms a step, here 3.28)
+    // barriers between order the threads, not the two ways of writing).  Plane q is written in iteration q - 1
+    // and its slot refilled from iteration q + 3 on, so one fence in four iterations is enough, at an
+    // iteration's end: right after the writes it waited for the loads in flight (256 x 256 x 128 FP64 3.35 ms
+    // a step; at every iteration's end 3.28)
     const bool fence = tma && (has_bot || has_top) && h < 2 * CW;
-    auto fence_walls = [&]() {
-        if (fence) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    auto fence_walls = [&](int c) {
+        if (fence && (c & 3) == 3) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     };
-    if (frame) walls(ib - 1, sm.planeS);
+    if (frame) {
+        walls(ib - 1, sm.planeS);
+        fence_walls(3);   // written before the first iteration: three are left
+    }
     block_sync();
 
     // byte offsets of this thread's cells in the ring slots of planes c-2 .. c+2 and
@@ -751,7 +756,7 @@ __global__ void __launch_bounds__(NT + FR, NB)
             if (h < CW && c < ie) put_col(c + 2, h - 1, col);
             Y = Yn;
             coef = coefn;
-            fence_walls();
+            fence_walls(c);
             next_plane(c);
         }
         settle();
