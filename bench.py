@@ -176,9 +176,9 @@ def kernel_bytes(name, P, prec):
     h1 = (r.Ny - 1) // 2 + 1
     G = (r.Nz) * (r.Nx - 1) * h1 * 16          # spectral slab incl. the top-plane slice
     return {
-        "stage_fused": 17 * s * S / 4,
-        "stage_utau": 0,
-        "stage_bc": 0,
+        "stage_fused": 17 * s * S / 4,   # k_stage_march
+        "stage_utau": 0,                 # k_utau, before the first stage
+        "stage_bc": 0,                   # k_stage_edge
         # read u, v, w (+ top plane of p); write half spectrum
         "p_rhs_ffty": 3 * s * N + G,
         "p_fftx_fwd": 2 * G,
@@ -438,7 +438,7 @@ def run_ours(args):
             "config": workload_config(args.config, P, args.precision, world),
             "e2e": e2e, "gpu_launches": launches, "roofline": roofline, "step_roofline": step_roof,
             "kernels": kernels, "cpu_baseline": cpu, "clocks": clk, "fp64": fp64,
-            "stage_tile": "form %dx%d/%d (by precision and grid size)" % stage_tile,
+            "stage_tile": "block form named %dx%d/%d (by precision and grid size; its tile is fitted to the grid)" % stage_tile,
             "reference_gpu": None if (args.no_refgpu or world > 1) else reference_gpu_sample(args.config),
         }
         print(json.dumps(out), flush=True)

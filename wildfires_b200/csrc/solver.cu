@@ -940,6 +940,8 @@ void drop_graphs(wf_ctx *c)
         }
 }
 
+// kernel kinds of wf_profile_phases by the names callers know: stage_fused is k_stage_march,
+// stage_bc k_stage_edge, p_tridiag whichever vertical solver the grid takes
 const char *kPhaseNames[WF_NPHASES] = {"stage_utau", "stage_fused", "stage_bc", "p_rhs_ffty", "p_fftx_fwd",
                                        "p_tridiag", "p_fftx_inv", "p_iffty_out", "project"};
 
