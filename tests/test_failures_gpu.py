@@ -50,7 +50,7 @@ def test_every_refused_allocation_in_create_is_reported_and_cleaned_up(params_fr
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_a_plane_given_up_is_reported_by_the_next_call_that_waits(prec, params_from_text, monkeypatch):
-    """With a wait limit of 0 (WF_STAGE_WAIT) the stage kernel gives up every plane: the call that next
+    """With a wait limit of 0 (WF_STAGE_WAIT) the stage kernel gives up the first plane of every block: the call that next
     waits for the context reports it, once.  The grid's columns (16 planes) are copied by TMA."""
     from wildfires_b200 import Ensemble, Solver, _abi
     L, dp = _abi.lib(), C.POINTER(C.c_double)

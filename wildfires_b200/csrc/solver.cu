@@ -1154,7 +1154,7 @@ wf_status wf_create(const Parameters *P, int precision, wf_ctx **out)
     c->d_kerr = reinterpret_cast<int *>(c->d_diag + kDiagValues);
     e = cudaMemset(c->d_kerr, 0, sizeof(int));
     if (e != cudaSuccess) { set_error("wf_create: %s", cudaGetErrorString(e)); return fail(WF_ERR_CUDA); }
-    if (const char *env = getenv("WF_STAGE_WAIT")) c->plane_wait = std::max(atoi(env), 0);   // polls, to exercise the path
+    if (const char *env = getenv("WF_STAGE_WAIT")) c->plane_wait = std::max(atoi(env), 0);   // of the first plane, to exercise the path
     if (!(getenv("WF_NO_TMA") && atoi(getenv("WF_NO_TMA")))) {
         // for the tensor maps; without it the stage kernel copies its planes by cp.async
         cudaDriverEntryPointQueryResult q;

@@ -592,18 +592,25 @@ __global__ void __launch_bounds__(NT + FR, NB)
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    int lost = -1;   // slot whose plane did not arrive in time (+ 8 in the walk): flagged, no further fetches and waits
+    // polls of the waits after the first plane's: FP32 takes the constant, FP64 the argument, each for the
+    // fewer spills
+    const int wait = E == 4 ? kPlaneWaitLimit : a.plane_wait;
+    // Parities of the slots' next arrivals; when a plane did not arrive in time, kLost and its slot (+ 8 in
+    // the walk) in the second byte: flagged, no further fetches and waits.  In one register: a word
+    // more spilled 48 bytes in the FP32 form with rows of 24, a limit from the arguments 16 (3 to 4% of an
+    // ensemble's step).
+    constexpr uint32_t kLost = 0x80000000u;
+    uint32_t phases = 0;
     auto fetch = [&](int c, int slot) {
         if (!tma) fetch_copy(c, slot);
-        else if (lost < 0) fetch_box(c, slot);
+        else if (!(phases & kLost)) fetch_box(c, slot);
     };
-    uint32_t phases = 0;
-    auto arrived = [&](int slot, int walk) {
-        if (tma && lost < 0) {
-            if (mbar_wait(sbase + sm.bar + slot * 8, (phases >> slot) & 1, a.plane_wait)) {
+    auto arrived = [&](int slot, int walk, int limit) {
+        if (tma && !(phases & kLost)) {
+            if (mbar_wait(sbase + sm.bar + slot * 8, (phases >> slot) & 1, limit)) {
                 phases ^= 1u << slot;
             } else {
-                lost = slot + walk;
+                phases |= kLost | (uint32_t)(slot + walk) << 8;
                 if (a.kerr) *(volatile int *)a.kerr = 1;
             }
         }
@@ -611,7 +618,8 @@ __global__ void __launch_bounds__(NT + FR, NB)
     // the thread that fetches gives the planes still due a bounded chance to land before the block gives up
     // its shared memory: of the first four those not waited for, in the walk the one
     auto settle = [&]() {
-        if (lost >= 0 && issuer)
+        const int lost = (phases >> 8) & 15;
+        if ((phases & kLost) && issuer)
             for (int r = lost & 7; r <= (lost < 8 ? 3 : lost & 7); r++)
                 mbar_wait(sbase + sm.bar + r * 8, (phases >> r) & 1, kPlaneWaitLimit);
     };
@@ -625,7 +633,8 @@ __global__ void __launch_bounds__(NT + FR, NB)
         for (int n = 0; n < 3; n++) put_col(ib - 2 + n, h - 1, q[n]);
     }
     if (!tma) asm volatile("cp.async.wait_group 0;" ::: "memory");
-    for (int r = 0; r < 4; r++) arrived(r, 0);
+    arrived(0, 0, a.plane_wait);
+    for (int r = 1; r < 4; r++) arrived(r, 0, wait);
     block_sync();
     V Y = fuel_at(ib - 1), coef = coef_at(ib - 1);
 
@@ -657,9 +666,8 @@ __global__ void __launch_bounds__(NT + FR, NB)
     // and its slot refilled from iteration q + 3 on, so one fence in four iterations is enough, at an
     // iteration's end: right after the writes it waited for the loads in flight (256 x 256 x 128 FP64 3.35 ms
     // a step; at every iteration's end 3.28)
-    const bool fence = tma && (has_bot || has_top) && h < 2 * CW;
     auto fence_walls = [&](int c) {
-        if (fence && (c & 3) == 3) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (tma && (has_bot || has_top) && h < 2 * CW && (c & 3) == 3) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     };
     if (frame) {
         walls(ib - 1, sm.planeS);
@@ -676,7 +684,7 @@ __global__ void __launch_bounds__(NT + FR, NB)
     auto next_plane = [&](int c) {
         // the plane fetched in this iteration (c + 3) is used from the next one on
         if (!tma) asm volatile("cp.async.wait_group 0;" ::: "memory");
-        if (c + 3 <= ie + 1) arrived(rn, 8);
+        if (c + 3 <= ie + 1) arrived(rn, 8, wait);
         rn = rn == SM::RS - 1 ? 0 : rn + 1;
         am2 = am1;
         am1 = a0;

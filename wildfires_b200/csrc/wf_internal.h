@@ -143,7 +143,7 @@ struct StageArgs {
     // host copies of the TMA tensor maps (CUtensorMap) of X, by tiles and by rows; nullptr: planes copied by cp.async
     const void *tmap[2];
     int *kerr;             // set by a stage kernel whose bounded wait for a plane gave up
-    int plane_wait;        // polls of each wait for a plane
+    int plane_wait;        // polls of the wait for a block's first plane, in FP64 for all (kPlaneWaitLimit but in tests)
 };
 constexpr int kPlaneWaitLimit = 1 << 20;   // polls before a plane is given up (about a second)
 
